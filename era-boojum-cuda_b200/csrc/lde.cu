@@ -39,7 +39,6 @@ __global__ void __launch_bounds__(256, BC_TOP_MIN_BLOCKS) lde_top_kernel(const L
   top_body<K, C>(p, blockIdx.x, blockIdx.y, smem);
 }
 
-typedef void (*TopKernel)(const LdeTopParams);
 typedef void (*PassKernelT)(const PassParams);
 
 static TopKernel pick_top(int K, int C);
@@ -140,6 +139,11 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
   const uint32_t nb = 1u << log_blowup;
   uint64_t *T = out + (uint64_t)(nb - 1) * coset_stride;
   const int np = pl.npasses;
+  // the top window runs on the tensor cores when every inverse pass below it
+  // does: those then apply n^-1 and the low bits' share of g^i (SHARE_G)
+  bool tc_top = !full_tile && np > 1 && tc_top_ok(pl.pass[0].K, log_n - pl.pass[0].K, log_blowup);
+  for (int i = 1; tc_top && i < np; i++)
+    tc_top = tc_window_ok(pl.pass[i].K, plan_lb(pl, log_n, i), num_cols, true, true);
   // A: inverse passes below the top window, bottom-up: in -> T
   for (int s = 0; s < np - 1; s++) {
     const int i = np - 1 - s;
@@ -156,11 +160,17 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     q.lb = plan_lb(pl, log_n, i);
     q.inverse = true;
     q.full_tile = full_tile;
+    if (tc_top) {
+      q.share = SHARE_G;
+      q.store_scale = s == 0; // n^-1
+    }
     LdeStep st;
     st.K = q.K;
     st.C = q.C;
     st.b2n = true;
     st.occ = pl.knobs.occ;
+    st.tc = q.tc = !full_tile && tc_pass_ok(q);
+    q.overlap = !full_tile && !steps.empty() && steps.back().tc;
     if (!build_pass(q, pass_walk, st.pass, st.grid, st.threads, st.smem)) return false;
     steps.push_back(st);
   }
@@ -181,7 +191,7 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     p.log_n = log_n;
     p.lb = log_n - K;
     p.log_blowup = log_blowup;
-    const uint32_t wc_log = (uint32_t)K + ilog2_ceil((uint32_t)C);
+    const uint32_t wc_log = tc_top ? 12 : (uint32_t)K + ilog2_ceil((uint32_t)C);
     p.log_g = full_tile ? (wc_log < 12 ? 12 - wc_log : 0) : choose_log_g(wc_log, num_cols);
     const uint32_t G = 1u << p.log_g;
     const uint64_t tiles = (1ull << log_n) >> wc_log;
@@ -196,6 +206,15 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     p.tabs = *tabs;
     const uint32_t tile = G << wc_log;
     st.threads = tile / 16;
+    if (tc_top) {
+      st.tc = true;
+      p.overlap = !full_tile && !steps.empty() && steps.back().tc ? 2 * (uint32_t)sm_count() : 0;
+      st.smem = tc_top_smem(K);
+      const uint64_t gy = (num_cols + p.cols_per_cta - 1) / p.cols_per_cta;
+      if (gy > 65535 || tiles > 0x7fffffffull) return false;
+      st.grid = dim3((uint32_t)tiles, (uint32_t)gy);
+      steps.push_back(st);
+    } else {
     const uint32_t nb = 1u << log_blowup;
     // forward power tables: all resident if they fit with two CTAs per SM, else
     // two slots fed ahead by cp.async from the precomputed ones, else refilled
@@ -253,6 +272,7 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     if (gy > 65535 || tiles > 0x7fffffffull) return false;
     st.grid = dim3((uint32_t)tiles, (uint32_t)gy);
     steps.push_back(st);
+    }
   }
   // C: forward passes below the top window for all cosets (column groups with prefix brev(k))
   for (int i = 1; i < np; i++) {
@@ -277,6 +297,8 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     st.K = q.K;
     st.C = q.C;
     st.occ = pl.knobs.occ;
+    st.tc = q.tc = !full_tile && tc_pass_ok(q);
+    q.overlap = !full_tile && !steps.empty() && steps.back().tc;
     if (!build_pass(q, pass_walk, st.pass, st.grid, st.threads, st.smem)) return false;
     steps.push_back(st);
   }
@@ -285,20 +307,23 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
 
 cudaError_t launch_lde_step(const LdeStep &st, cudaStream_t stream) {
   if (st.top) {
-    TopKernel kern = pick_top(st.K, st.C);
+    TopKernel kern = st.tc ? pick_top_tc(st.K) : pick_top(st.K, st.C);
     if (!kern) return cudaErrorInvalidValue;
     if (st.smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st.smem);
       if (e != cudaSuccess) return e;
     }
+    if (st.tc) return launch_tc(kern, st.grid, st.smem, st.topp, st.topp.overlap != 0, stream);
     kern<<<st.grid, st.threads, st.smem, stream>>>(st.topp);
   } else {
-    PassKernel kern = pick_pass_kernel(st.K, st.C, st.b2n, st.pass.inverse != 0, st.occ);
+    PassKernel kern = st.tc ? pick_pass_kernel_tc(st.K, st.pass.lb == 0, st.b2n, st.pass.inverse != 0)
+                            : pick_pass_kernel(st.K, st.C, st.b2n, st.pass.inverse != 0, st.occ);
     if (!kern) return cudaErrorInvalidValue;
     if (st.smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st.smem);
       if (e != cudaSuccess) return e;
     }
+    if (st.tc) return launch_tc(kern, st.grid, st.smem, st.pass, st.pass.overlap != 0, stream);
     kern<<<st.grid, st.threads, st.smem, stream>>>(st.pass);
   }
   return cudaGetLastError();

@@ -55,6 +55,7 @@ struct LdeTopParams {
   uint32_t fwd_mode;
   const uint64_t *fwd_tables; // precomputed forward tables of the cosets (or nullptr)
   const uint64_t *inv_table;  // precomputed inverse table (or nullptr)
+  uint32_t overlap;           // tensor-core kernel: CTAs of one wave when launched beside its predecessor's end, else 0
   uint32_t dbuf;              // two tiles, the next column group copied (cp.async) during this one;
                               // honoured by the 8-column kernels only (C == 8)
   uint32_t scale_off;         // windows of 4 bits or more: word offset in shared memory of the
@@ -632,12 +633,20 @@ __host__ __device__ constexpr uint32_t top_smem_words(uint32_t tile, int K, uint
 // (98 KB), which keeps two CTAs on an SM and fits the persistent kernel.
 constexpr uint32_t TOP_RESIDENT_SMEM_MAX = top_smem_words(4096, 12, 1) * 8;
 
+typedef void (*TopKernel)(const LdeTopParams);
+// The tensor-core top-window kernels (lde_tc.cu): 256 threads, 4096-element
+// tiles; their inverse passes below must be tensor-core ones (SHARE_G).
+TopKernel pick_top_tc(int K);
+size_t tc_top_smem(int K);
+bool tc_top_ok(int K, uint32_t lb, uint32_t log_blowup);
+
 // One kernel of a fused LDE: either a pass (ntt_pass_kernel) or the top-window
 // kernel, with its parameters and launch shape.
 struct LdeStep {
   bool top = false;
   int K = 0, C = 1;
   bool b2n = false;
+  bool tc = false; // the tensor-core kernel
   int occ = 0; // occupancy variant of a pass kernel (Knobs::occ)
   PassParams pass{};
   LdeTopParams topp{};

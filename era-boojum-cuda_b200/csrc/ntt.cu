@@ -47,6 +47,7 @@ struct DeviceCtx {
   uint64_t *block = nullptr;
   uint64_t *top_pw = nullptr; // precomputed top-window power tables
   uint64_t *top_pw_st = nullptr; // the same for the short-round-on-top partition
+  uint8_t *tc = nullptr; // tensor-core matrices, then the wait-error word
   DevTables tabs{};
   int sms = 0;
 };
@@ -178,12 +179,19 @@ cudaError_t context_create_current() {
   if (e == cudaSuccess) e = cudaMalloc(&c.top_pw_st, top_pw_words() * sizeof(uint64_t));
   if (e == cudaSuccess) e = top_pw_fill<1, 0>(c.tabs, c.top_pw);
   if (e == cudaSuccess) e = top_pw_fill<1, 1>(c.tabs, c.top_pw_st);
+  if (e == cudaSuccess) e = cudaMalloc(&c.tc, tc_table_bytes() + 16);
+  if (e == cudaSuccess) e = cudaMemset(c.tc + tc_table_bytes(), 0, 16);
+  if (e == cudaSuccess) e = tc_fill_tables(c.tc, c.tabs);
+  c.tabs.tc_img = c.tc;
+  c.tabs.wait_error = reinterpret_cast<uint32_t *>(c.tc + tc_table_bytes());
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     cudaFree(c.block);
     cudaFree(c.top_pw);
     cudaFree(c.top_pw_st);
+    cudaFree(c.tc);
     c.block = c.top_pw = c.top_pw_st = nullptr;
+    c.tc = nullptr;
     return e;
   }
   cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, d);
@@ -210,9 +218,12 @@ cudaError_t context_destroy_current() {
   cudaError_t e = cudaFree(c.block);
   const cudaError_t e2 = cudaFree(c.top_pw);
   const cudaError_t e3 = cudaFree(c.top_pw_st);
+  const cudaError_t e4 = cudaFree(c.tc);
   if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = e3;
+  if (e == cudaSuccess) e = e4;
   c.block = c.top_pw = c.top_pw_st = nullptr;
+  c.tc = nullptr;
   return e;
 }
 
@@ -391,8 +402,9 @@ bool build_pass(const PassLaunch &pl, int cols_factor_max, PassParams &p, dim3 &
   p.log_groups = pl.log_groups;
   p.log_n = pl.log_n;
   p.lb = pl.lb;
-  const uint32_t wc_log = (uint32_t)K + log2_ceil((uint32_t)C);
-  p.log_g = pl.full_tile ? (wc_log < 12 ? 12 - wc_log : 0) : choose_log_g(wc_log, pl.cols);
+  // window and run of a tile, log2; tensor-core tiles fill up with low positions, then columns
+  const uint32_t wc_log = pl.tc ? 12 - tc_log_g(K, pl.lb == 0) : (uint32_t)K + log2_ceil((uint32_t)C);
+  p.log_g = pl.full_tile || pl.tc ? (wc_log < 12 ? 12 - wc_log : 0) : choose_log_g(wc_log, pl.cols);
   const uint32_t G = 1u << p.log_g;
   const uint64_t tiles_per_col = (1ull << pl.log_n) >> wc_log;
   const uint64_t groups = 1ull << pl.log_groups;
@@ -406,6 +418,8 @@ bool build_pass(const PassLaunch &pl, int cols_factor_max, PassParams &p, dim3 &
   p.load_scale = pl.load_scale;
   p.store_scale = pl.store_scale;
   p.canon_out = pl.canon_out;
+  p.share = pl.share;
+  p.overlap = pl.overlap ? 2 * (uint32_t)sm_count() : 0;
   p.has_coset = pl.has_coset;
   p.coset_kshift = pl.coset_kshift;
   p.vec_in = ((uintptr_t)p.in % 16 == 0 && p.stride_in % 2 == 0 && p.group_stride_in % 2 == 0) ? 1 : 0;
@@ -413,7 +427,7 @@ bool build_pass(const PassLaunch &pl, int cols_factor_max, PassParams &p, dim3 &
   p.tabs = *tabs;
   const uint32_t tile = G << wc_log;
   threads = tile / 16;
-  smem_bytes = (size_t)pass_smem_words(tile, K) * sizeof(uint64_t);
+  smem_bytes = pl.tc ? tc_pass_smem(K) : (size_t)pass_smem_words(tile, K) * sizeof(uint64_t);
   const uint64_t gy = groups * p.chunks_per_group;
   if (tiles_per_col > 0x7fffffffull || gy > 65535) return false;
   grid = dim3((uint32_t)tiles_per_col, (uint32_t)gy);
@@ -428,12 +442,14 @@ cudaError_t launch_pass(const PassLaunch &pl, cudaStream_t stream) {
   uint32_t threads;
   size_t smem;
   if (!build_pass(pl, pl.walk, p, grid, threads, smem)) return cudaErrorInvalidConfiguration;
-  PassKernel kern = pick_pass_kernel(pl.K, pl.C, pl.b2n, pl.inverse, pl.occ);
+  PassKernel kern = pl.tc ? pick_pass_kernel_tc(pl.K, pl.lb == 0, pl.b2n, pl.inverse)
+                          : pick_pass_kernel(pl.K, pl.C, pl.b2n, pl.inverse, pl.occ);
   if (!kern) return cudaErrorInvalidValue;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
+  if (pl.tc) return launch_tc(kern, grid, smem, p, pl.overlap, stream);
   kern<<<grid, threads, smem, stream>>>(p);
   return cudaGetLastError();
 }
@@ -443,6 +459,14 @@ cudaError_t launch_ntt(const Plan &pl, const uint64_t *in, uint64_t *out, uint32
                        uint32_t coset_idx, cudaStream_t stream) {
   if (!device_tables()) return cudaErrorInitializationError;
   if (num_ntts == 0) return cudaSuccess;
+  // a coset transform's scaling is shared by its passes when all of them run on
+  // the tensor cores, and otherwise applied whole by its first (forward) or
+  // last (inverse) pass
+  const bool scaled = log_ext > 0 && bitrev_inputs == inverse;
+  bool share = scaled;
+  for (int i = 0; share && i < pl.npasses; i++)
+    share = tc_window_ok(pl.pass[i].K, plan_lb(pl, log_n, i), num_ntts, bitrev_inputs, inverse);
+  bool prev_tc = false;
   for (int s = 0; s < pl.npasses; s++) {
     const int i = bitrev_inputs ? pl.npasses - 1 - s : s; // b2n runs the passes bottom-up
     const bool first = s == 0, last = s == pl.npasses - 1;
@@ -458,13 +482,16 @@ cudaError_t launch_ntt(const Plan &pl, const uint64_t *in, uint64_t *out, uint32
     q.log_n = log_n;
     q.lb = plan_lb(pl, log_n, i);
     q.inverse = inverse;
-    q.load_scale = first && !inverse && log_ext > 0;
+    q.load_scale = first && !inverse && log_ext > 0 && !share;
+    q.share = share ? (inverse ? SHARE_COSET_INV : SHARE_COSET) : SHARE_NONE;
     q.store_scale = last && inverse;
     q.canon_out = last;
     q.has_coset = log_ext > 0 ? 1 : 0;
     q.coset_kshift = coset_idx ? coset_idx << (PW_LOG - log_n - log_ext) : 0;
     q.walk = plan_walk(pl);
     q.occ = pl.knobs.occ;
+    q.overlap = prev_tc;
+    prev_tc = q.tc = tc_pass_ok(q);
     cudaError_t e = launch_pass(q, stream);
     if (e != cudaSuccess) return e;
   }

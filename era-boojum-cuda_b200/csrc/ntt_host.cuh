@@ -72,6 +72,12 @@ Plan default_plan(uint32_t log_n);
 Plan tuned_plan(uint32_t log_n, uint32_t log_blowup);
 bool plan_valid(const Plan &pl, uint32_t log_n);
 
+// Scaling by base^i, i the natural index, spread over the passes: the index is
+// the sum of its windows' bit fields, and a tensor-core pass applies its own
+// window's share at no cost (ntt_tc.cuh), so every pass of a transform has
+// the same setting.  The base: the coset's c, c^-1, or g.
+enum : uint32_t { SHARE_NONE = 0, SHARE_COSET = 1, SHARE_COSET_INV = 2, SHARE_G = 3 };
+
 // One pass over columns that may come in 2^log_groups groups (see ntt_pass.cuh).
 struct PassLaunch {
   int K = 0, C = 1;
@@ -86,6 +92,9 @@ struct PassLaunch {
   bool inverse = false, load_scale = false, store_scale = false, canon_out = false;
   uint32_t has_coset = 0, coset_kshift = 0;
   bool full_tile = false; // always 4096-element tiles (256 threads), as the batch kernel runs them
+  bool tc = false;        // the tensor-core kernel (needs tc_pass_ok)
+  uint32_t share = 0;     // tc only: SHARE_*
+  bool overlap = false;   // tc only: its predecessor in the stream is a tensor-core kernel of the same call
   int walk = BC_COLS_FACTOR_MAX, occ = 0; // column-group walk cap; occupancy variant (Knobs)
 };
 cudaError_t launch_pass(const PassLaunch &pl, cudaStream_t stream);
@@ -101,6 +110,35 @@ typedef void (*PassKernel)(const PassParams);
 // when not instantiated); occ (Knobs::occ) selects the occupancy variant of the
 // C = 1 kernels of 9..12 bits, 0 the default one.
 PassKernel pick_pass_kernel(int K, int C, bool b2n, bool inverse, int occ = 0);
+// The tensor-core form of the same passes (ntt_tc.cu): 256 threads, tiles of
+// 4096 elements, tc_pass_smem bytes of shared memory; low: the window starts
+// at bit 0.  tc_window_ok / tc_pass_ok: whether a window / a pass runs on it.
+PassKernel pick_pass_kernel_tc(int K, bool low, bool b2n, bool inverse);
+size_t tc_pass_smem(int K);
+uint32_t tc_log_g(int K, bool low);
+bool tc_window_ok(int K, uint32_t lb, uint32_t cols, bool b2n, bool inverse);
+bool tc_pass_ok(const PassLaunch &q);
+// Constant matrices of its rounds and the tables of the tensor-core top-window
+// kernel behind them (DevTables::tc_img; lde_tc.cu).
+size_t tc_table_bytes();
+cudaError_t tc_fill_images(uint8_t *img);
+cudaError_t tc_fill_tables(uint8_t *img, const DevTables &tabs);
+// Launches a tensor-core kernel; overlap: beside the end of its predecessor,
+// which must be a tensor-core kernel too (tc.cuh, wait_previous).
+template <class P>
+cudaError_t launch_tc(void (*kern)(const P), dim3 grid, size_t smem, const P &p, bool overlap, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
 // Column-group walk caps of a plan's passes and top-window kernel.
 inline int plan_walk(const Plan &pl) { return pl.knobs.walk ? pl.knobs.walk : BC_COLS_FACTOR_MAX; }
 inline int plan_top_walk(const Plan &pl) { return pl.knobs.top_walk ? pl.knobs.top_walk : BC_TOP_COLS_FACTOR_MAX; }

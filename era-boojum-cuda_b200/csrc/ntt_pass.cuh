@@ -86,6 +86,8 @@ struct PassParams {
   uint32_t coset_kshift; // coset_idx << (PW_LOG - log_n - log_ext)
   uint32_t vec_in;       // 16-byte loads allowed (alignment checked on the host)
   uint32_t vec_out;      // 16-byte stores allowed
+  uint32_t overlap;      // tensor-core passes only: CTAs of one wave when launched beside its predecessor's end, else 0
+  uint32_t share;        // tensor-core passes only (SHARE_*): scale by this window's share of base^i
   DevTables tabs;
 };
 

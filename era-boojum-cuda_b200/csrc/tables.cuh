@@ -59,6 +59,8 @@ struct DevTables {
   const uint64_t *w_lo[2];  // [0] w^e, [1] w^-e  with w = w_{2^PW_LOG}
   const uint64_t *w_hi[2];
   uint64_t inv_pow2[TW_LOG + 1]; // 2^-k
+  const uint8_t *tc_img; // matrices of the tensor-core rounds (tc.cuh, img_index)
+  uint32_t *wait_error;  // set by a kernel whose bounded completion wait ran out
 };
 
 } // namespace bc

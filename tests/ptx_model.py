@@ -140,6 +140,8 @@ def run(block, inputs: list[int], outputs: int = 1):
         elif base in ("mad", "madc"):
             prod = (a[0] & M32) * (a[1] & M32)
             if "wide" in flags:
+                if "s32" in flags:
+                    prod = ((a[0] & M32 ^ 1 << 31) - (1 << 31)) * ((a[1] & M32 ^ 1 << 31) - (1 << 31))
                 regs[d] = (prod + a[2]) & M64
                 continue
             part = (prod >> 32) & M32 if "hi" in flags else prod & M32

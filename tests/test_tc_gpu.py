@@ -1,0 +1,122 @@
+"""The tensor-core passes and top windows against the oracle, at the sizes where
+their tiles, rounds and scalings change: every window size at both ends of the
+index, short rounds, column counts around a tile's, cosets, odd strides."""
+import numpy as np
+import pytest
+
+from conftest import raw_u64, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+
+def _ntt(log_n, cols, bitrev, inverse, ext=0, coset=0, gap=0, plan=None, seed=0):
+    import torch
+
+    import bc_ntt
+    import oracle
+
+    rng = np.random.default_rng(seed + 1000 * log_n + cols)
+    n, stride = 1 << log_n, (1 << log_n) + gap
+    x = raw_u64(rng, cols * stride)
+    x[: min(n, 64)] = 2**64 - 1  # the largest digit sums
+    d, o = to_dev(x), torch.full((cols * stride,), 7, dtype=torch.int64, device="cuda")
+    if plan:
+        bc_ntt.batch_ntt_with_plan(d, o, log_n, cols, stride, stride, bitrev, inverse, ext, coset, plan)
+    else:
+        bc_ntt.batch_ntt_internal(d.data_ptr(), o.data_ptr(), log_n, cols, stride, stride, bitrev, inverse, ext, coset)
+    exp = np.asarray(oracle.batch_ntt(x, log_n, cols, stride, stride, bitrev, inverse, ext, coset))
+    got = to_host(o).reshape(cols, stride)
+    assert np.array_equal(got[:, :n], exp.reshape(cols, stride)[:, :n])
+    assert (got[:, n:] == 7).all()
+
+
+@pytest.mark.parametrize("log_n", [8, 9, 10, 11, 12])
+@pytest.mark.parametrize("bitrev,inverse", [(False, False), (False, True), (True, False), (True, True)])
+def test_low_windows(gpu_ctx, log_n, bitrev, inverse):
+    g = 1 << (12 - log_n)  # columns of a tile
+    for cols in {1, max(1, g - 1), g, g + max(1, 3 * g // 4), 2 * g + 1}:
+        _ntt(log_n, cols, bitrev, inverse)
+    _ntt(log_n, g, bitrev, inverse, gap=3)
+    if bitrev == inverse:
+        _ntt(log_n, g, bitrev, inverse, ext=2, coset=3, gap=1)
+
+
+PLANS = [[(4, 8), (8, 1)], [(5, 8), (9, 1)], [(8, 8), (8, 1)], [(9, 8), (8, 1)], [(10, 4), (9, 1)], [(8, 8), (12, 1)],
+         [(4, 8), (8, 8), (8, 1)], [(11, 2), (8, 1)]]
+
+
+@pytest.mark.parametrize("plan", PLANS, ids=lambda p: "+".join(f"{k}.{c}" for k, c in p))
+@pytest.mark.parametrize("bitrev,inverse", [(False, False), (False, True), (True, False), (True, True)])
+def test_window_plans(gpu_ctx, plan, bitrev, inverse):
+    log_n = sum(k for k, _ in plan)
+    for cols, gap in ((1, 0), (9 if log_n < 19 else 3, 5)):
+        _ntt(log_n, cols, bitrev, inverse, gap=gap, plan=plan)
+        if bitrev == inverse:  # the scaling by the coset's powers, shared by the passes where all are of one kind
+            _ntt(log_n, cols, bitrev, inverse, ext=1, coset=1, gap=gap, plan=plan)
+
+
+@pytest.mark.parametrize("plan", [[(4, 8), (8, 1)], [(5, 8), (8, 1)], [(8, 8), (8, 1)], [(10, 4), (8, 1)],
+                                  [(4, 8), (4, 8), (8, 1)], [(5, 8), (4, 8), (9, 1)]],
+                         ids=lambda p: "+".join(f"{k}.{c}" for k, c in p))
+@pytest.mark.parametrize("log_b", [1, 3, 5])
+def test_lde_top_windows(gpu_ctx, plan, log_b):
+    import torch
+
+    import bc_ntt
+    import oracle
+
+    log_n = sum(k for k, _ in plan)
+    text = f"{log_n} {log_b} {len(plan)} " + " ".join(f"{k} {c}" for k, c in plan) + "\n"
+    old = bc_ntt.plan_table_export()
+    try:
+        bc_ntt.plan_table_import(text)
+        for cols in ((1, 13) if log_n + log_b < 20 else (3,)):
+            n = 1 << log_n
+            x = raw_u64(np.random.default_rng(log_n + cols), cols * n)
+            x[:64] = 2**64 - 1
+            d, o = to_dev(x), torch.zeros(cols * n << log_b, dtype=torch.int64, device="cuda")
+            bc_ntt.lde(d, o, log_n, cols, log_b)
+            assert np.array_equal(to_host(o), oracle.lde(x, log_n, cols, n, log_b)), cols
+    finally:
+        bc_ntt.plan_table_clear()
+        if old:
+            bc_ntt.plan_table_import(old)
+
+
+def test_chains_in_a_graph_and_on_two_streams(gpu_ctx):
+    """Kernels of one call overlap each other's start: repeated calls that read the previous call's output, two
+    streams at once, and a captured graph give what single calls give."""
+    import torch
+
+    import bc_ntt
+
+    log_n, cols = 16, 16
+    n = 1 << log_n
+    x = to_dev(raw_u64(np.random.default_rng(3), cols * n))
+
+    def there_and_back(a, b):
+        bc_ntt.batch_ntt_internal(a.data_ptr(), b.data_ptr(), log_n, cols, n, n, False, False, 0, 0)
+        bc_ntt.batch_ntt_internal(b.data_ptr(), a.data_ptr(), log_n, cols, n, n, True, True, 0, 0)
+
+    a0, b0 = x.clone(), torch.empty_like(x)
+    there_and_back(a0, b0)
+    torch.cuda.synchronize()
+    want = to_host(a0)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    bufs = [(x.clone(), torch.empty_like(x)) for _ in streams]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, (a, b) in zip(streams, bufs):
+            with torch.cuda.stream(s):
+                there_and_back(a, b)
+    torch.cuda.synchronize()
+    for a, _ in bufs:
+        assert np.array_equal(to_host(a), want)
+    a, b = x.clone(), torch.empty_like(x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        there_and_back(a, b)
+    for _ in range(5):
+        g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(to_host(a), want)
