@@ -141,7 +141,7 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
   const int np = pl.npasses;
   // the top window runs on the tensor cores when every inverse pass below it
   // does: those then apply n^-1 and the low bits' share of g^i (SHARE_G)
-  bool tc_top = !full_tile && np > 1 && tc_top_ok(pl.pass[0].K, log_n - pl.pass[0].K, log_blowup);
+  bool tc_top = np > 1 && tc_top_ok(pl.pass[0].K, log_n - pl.pass[0].K, log_blowup);
   for (int i = 1; tc_top && i < np; i++)
     tc_top = tc_window_ok(pl.pass[i].K, plan_lb(pl, log_n, i), num_cols, true, true);
   // A: inverse passes below the top window, bottom-up: in -> T
@@ -169,7 +169,7 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     st.C = q.C;
     st.b2n = true;
     st.occ = pl.knobs.occ;
-    st.tc = q.tc = !full_tile && tc_pass_ok(q);
+    st.tc = q.tc = tc_pass_ok(q);
     q.overlap = !full_tile && !steps.empty() && steps.back().tc;
     if (!build_pass(q, pass_walk, st.pass, st.grid, st.threads, st.smem)) return false;
     steps.push_back(st);
@@ -297,7 +297,7 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
     st.K = q.K;
     st.C = q.C;
     st.occ = pl.knobs.occ;
-    st.tc = q.tc = !full_tile && tc_pass_ok(q);
+    st.tc = q.tc = tc_pass_ok(q);
     q.overlap = !full_tile && !steps.empty() && steps.back().tc;
     if (!build_pass(q, pass_walk, st.pass, st.grid, st.threads, st.smem)) return false;
     steps.push_back(st);

@@ -33,6 +33,7 @@
 
 #include "../../include/bc_ntt.h"
 #include "lde.cuh"
+#include "lde_tc.cuh"
 
 namespace bc {
 
@@ -46,7 +47,7 @@ struct BatchRecord {
   uint32_t shape;
   int32_t pred;     // record that must be complete before any item of this one, or -1
   uint32_t n_items; // CTAs of this kernel
-  uint32_t pad;
+  uint32_t tc;      // a tensor-core body: shape is a tc_shape_id
   union {
     PassParams pass;
     LdeTopParams top;
@@ -59,7 +60,11 @@ __host__ __device__ constexpr uint64_t make_item(uint32_t rec, uint32_t by, uint
 }
 
 constexpr uint32_t BATCH_THREADS = 256;
-constexpr uint32_t BATCH_SMEM_BYTES = TOP_RESIDENT_SMEM_MAX; // largest body: top window of 12 bits, one forward table
+// largest bodies: the top window of 12 bits with one forward table, and the
+// tensor-core top window of 10 bits (two CTAs an SM either way)
+constexpr uint32_t BATCH_SMEM_BYTES = TOP_RESIDENT_SMEM_MAX > tc::top_tc_smem_bytes<10, true>()
+                                          ? TOP_RESIDENT_SMEM_MAX
+                                          : tc::top_tc_smem_bytes<10, true>();
 
 // The bodies the persistent kernel can run: every window shape of the default
 // plans (and of the tuner's candidates).
@@ -102,13 +107,65 @@ __device__ __forceinline__ void run_body(const BatchRecord &rec, uint32_t bx, ui
   }
 }
 
+// The tensor-core bodies: top windows, and the inverse (b2n) and forward passes
+// of windows at bit 0 (low) and above.
+__host__ __device__ constexpr uint32_t tc_shape_id(bool top, bool b2n, bool low, int K) {
+  return (top ? 1u << 7 : 0u) | (b2n ? 1u << 6 : 0u) | (low ? 1u << 5 : 0u) | (uint32_t)K;
+}
+#define BC_BATCH_TC_TOPS(X) X(4, false) X(5, true) X(8, false) X(10, true)
+#define BC_BATCH_TC_PASSES(X)                                                                                        \
+  X(true, true, 8) X(true, true, 9) X(true, true, 10) X(true, true, 11) X(true, true, 12) X(false, true, 8)         \
+  X(false, true, 9) X(false, true, 10) X(false, true, 11) X(false, true, 12) X(true, false, 8) X(true, false, 9)    \
+  X(true, false, 10) X(false, false, 8) X(false, false, 9) X(false, false, 10)
+
+bool batch_tc_shape_supported(uint32_t id) {
+#define BC_CASE(K, WIDE)                                                                                             \
+  if (id == tc_shape_id(true, false, false, K)) return true;
+  BC_BATCH_TC_TOPS(BC_CASE)
+#undef BC_CASE
+#define BC_CASE(B2N, LOW, K)                                                                                         \
+  if (id == tc_shape_id(false, B2N, LOW, K)) return true;
+  BC_BATCH_TC_PASSES(BC_CASE)
+#undef BC_CASE
+  return false;
+}
+
+template <int K, bool WIDE>
+__device__ __noinline__ void run_tc_top(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
+  tc::top_body_tc<K, WIDE>(rec.u.top, bx, by, smem, ctx, false);
+}
+template <bool B2N, bool LOW, int K>
+__device__ __noinline__ void run_tc_pass(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
+  tc::pass_body_tc<K, LOW, B2N, B2N>(rec.u.pass, bx, by, smem, ctx, false);
+}
+
+__device__ __forceinline__ void run_tc_body(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem,
+                                            tc::Ctx &ctx) {
+  switch (rec.shape) {
+#define BC_CASE(K, WIDE)                                                                                             \
+  case tc_shape_id(true, false, false, K):                                                                           \
+    run_tc_top<K, WIDE>(rec, bx, by, smem, ctx);                                                                     \
+    break;
+    BC_BATCH_TC_TOPS(BC_CASE)
+#undef BC_CASE
+#define BC_CASE(B2N, LOW, K)                                                                                         \
+  case tc_shape_id(false, B2N, LOW, K):                                                                              \
+    run_tc_pass<B2N, LOW, K>(rec, bx, by, smem, ctx);                                                                \
+    break;
+    BC_BATCH_TC_PASSES(BC_CASE)
+#undef BC_CASE
+  default:
+    break;
+  }
+}
+
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
-// status bit 0: a dependency wait expired (the batch's results are invalid).
+// status bit 0: a dependency wait expired, bit 1: a tensor-core completion wait did (the batch's results are invalid).
 // wait_limit: SM clock cycles one dependency wait may take (read once per CTA).
 __global__ void __launch_bounds__(BATCH_THREADS, 2)
     lde_batch_kernel(const BatchRecord *__restrict__ recs, const uint64_t *__restrict__ items, uint32_t n_items,
@@ -116,12 +173,15 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
   extern __shared__ uint64_t smem[];
   __shared__ uint32_t s_idx, s_ok;
   __shared__ BatchRecord s_rec; // the item's kernel parameters, read by the body from shared memory
+  __shared__ __align__(16) uint64_t s_tc[2]; // barrier and tensor-memory address of the tensor-core bodies
   const long long timeout_cycles = threadIdx.x == 0 ? *wait_limit : 0;
+  tc::Ctx ctx = tc::begin(s_tc);
+  uint8_t *const tc_smem = reinterpret_cast<uint8_t *>(smem) + ((1024 - (tc::smem_u32(smem) & 1023)) & 1023);
   for (;;) {
     if (threadIdx.x == 0) s_idx = atomicAdd(next, 1u);
     __syncthreads();
     const uint32_t idx = s_idx;
-    if (idx >= n_items) return;
+    if (idx >= n_items) break;
     const uint64_t it = items[idx];
     const uint32_t r = (uint32_t)(it >> 48), by = (uint32_t)(it >> 28) & 0xFFFFFu, bx = (uint32_t)it & 0xFFFFFFFu;
     const BatchRecord &rec = recs[r];
@@ -145,13 +205,20 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
       s_ok = ok;
     }
     __syncthreads();
-    if (s_ok) run_body(s_rec, bx, by, smem);
+    if (s_ok) {
+      if (s_rec.tc)
+        run_tc_body(s_rec, bx, by, tc_smem, ctx);
+      else
+        run_body(s_rec, bx, by, smem);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(done + r, 1u);
     }
   }
+  if (ctx.bad) atomicOr(status, 2u);
+  tc::end(ctx, nullptr);
 }
 
 } // namespace bc
@@ -250,7 +317,9 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
                            jb.coset_stride, jb.log_blowup, true, 16, 16, steps[j]))
         return false;
       for (const LdeStep &st : steps[j])
-        if (!batch_shape_supported(shape_id(st.top, st.b2n, st.K, st.C)) || st.threads != BATCH_THREADS ||
+        if (!(st.tc ? batch_tc_shape_supported(tc_shape_id(st.top, st.b2n, !st.top && st.pass.lb == 0, st.K))
+                    : batch_shape_supported(shape_id(st.top, st.b2n, st.K, st.C))) ||
+            st.threads != BATCH_THREADS ||
             st.smem > BATCH_SMEM_BYTES || st.grid.x >= (1u << 28) || st.grid.y >= (1u << 20) ||
             (!st.top && st.pass.inverse != (uint32_t)st.b2n)) // the kernel carries LDE passes only
           return false;
@@ -284,7 +353,9 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
       const LdeStep &st = steps[j][d];
       BatchRecord r;
       std::memset(&r, 0, sizeof(r));
-      r.shape = shape_id(st.top, st.b2n, st.K, st.C);
+      r.tc = st.tc;
+      r.shape = st.tc ? tc_shape_id(st.top, st.b2n, !st.top && st.pass.lb == 0, st.K)
+                      : shape_id(st.top, st.b2n, st.K, st.C);
       r.pred = last[j];
       r.n_items = st.grid.x * st.grid.y;
       if (st.top)
