@@ -221,15 +221,18 @@ __device__ __forceinline__ void top_body_tc(const LdeTopParams &p, uint32_t bx, 
   const uint32_t nb = 1u << p.log_blowup, step_bytes = 8u << p.lb;
   const uint8_t *gt = p.tabs.tc_img;
 
-  // operand words of the first round: straight from global memory
+  // operand words of the first round: each thread its row's 16, asynchronously
   const uint32_t e_in = top_in_elem<K, LC, WIDE, 0>(tid), a_in = top_addr<K, LC, WIDE, 0>(e_in);
-  uint64_t x[16];
   auto load = [&](uint32_t c0) {
     const uint64_t *src = elem_at<K, LC>(p.in + (uint64_t)c0 * p.stride_in + base_off, e_in, p.stride_in, step_bytes);
 #pragma unroll
-    for (uint32_t s = 0; s < 16; s++)
-      x[s] = __ldcg(elem_at<K, LC>(src, top_word_elem<K, LC, WIDE, 0>(s), p.stride_in, step_bytes));
+    for (uint32_t s = 0; s < 16; s++) {
+      const uint32_t es = top_word_elem<K, LC, WIDE, 0>(s);
+      cp_async8(tile + xor_part(a_in, top_addr<K, LC, WIDE, 0>(es)), elem_at<K, LC>(src, es, p.stride_in, step_bytes));
+    }
+    cp_async_commit();
   };
+
   if (!tables_first) {
     if (p.overlap) wait_previous();
     load(col_begin);
@@ -291,11 +294,7 @@ __device__ __forceinline__ void top_body_tc(const LdeTopParams &p, uint32_t bx, 
 #pragma unroll 1
   for (uint32_t c0 = col_begin; c0 < col_end; c0++) {
     const bool more = c0 + 1 < col_end;
-#pragma unroll
-    for (int s = 0; s < 16; s += 2)
-      *reinterpret_cast<ulonglong2 *>(tile + xor_part(a_in, top_addr<K, LC, WIDE, 0>(top_word_elem<K, LC, WIDE, 0>(s)))) =
-          make_ulonglong2(x[s], x[s + 1]);
-    if (WIDE && c0 == col_begin) cp_async_wait<0>();
+    cp_async_wait<0>();
     if constexpr (N == 2) { // inverse, bottom round
       top_multiply<WIDE>(ctx, t_tile, t_full);
       constexpr int FB = LC; // tile index bit of the field
@@ -341,7 +340,6 @@ __device__ __forceinline__ void top_body_tc(const LdeTopParams &p, uint32_t bx, 
         if (kn || more) fetch_coset(kn, slot ^ 1);
       }
       step++;
-      if (more && k + 1 == nb) load(c0 + 1);
       top_multiply<WIDE>(ctx, t_tile, WIDE ? t_full : t_full + (2 + slot) * IMG_BYTES);
       if constexpr (N == 2) { // top round to bottom round
         constexpr int FB = LC + K - LR;
@@ -358,6 +356,7 @@ __device__ __forceinline__ void top_body_tc(const LdeTopParams &p, uint32_t bx, 
         });
         top_multiply<WIDE>(ctx, t_tile, t_full);
       }
+      if (more && k + 1 == nb) load(c0 + 1); // the tile is free
       const uint32_t eo = top_out_elem<K, LC, WIDE, 2 * N - 1>(tid);
       uint64_t *dst = elem_at<K, LC>(p.out + (uint64_t)k * p.coset_stride + (uint64_t)c0 * p.stride_out + base_off, eo,
                                      p.stride_out, step_bytes);

@@ -243,48 +243,61 @@ __device__ __forceinline__ void pass_body_tc(const PassParams &p, uint32_t bx, u
   const uint32_t step_bytes = 8u << p.lb; // one window position
   // the thread's row in the first and the last round
   const uint32_t e_in = elem_of_row<K, LC, B2N, 0>(tid), e_out = elem_of_row<K, LC, B2N, LAST>(tid);
-  const uint32_t a_in = addr_of<K, LC, B2N, 0>(e_in), a_out = addr_of<K, LC, B2N, LAST>(e_out);
+  const uint32_t a_in = addr_of<K, LC, B2N, 0>(e_in);
 
-  // B2N over single positions copies its tile as it lies (cp.async); the others load words into registers
-  constexpr bool COPY_IN = B2N && LOW, COPY_OUT = !B2N && LOW;
-  auto copy_in = [&](uint32_t c0) {
+  // The tile of column group c0, asynchronously (cp.async): a window at bit 0 of
+  // a DIF pass as it lies, 16 bytes at a time; else each thread its row's 16
+  // words (neighbouring threads take neighbouring addresses).  Issued as soon as
+  // the last round's products are done, so it overlaps that round's folding and
+  // stores.  Slots of columns past the chunk keep what they hold: rows and
+  // diagonal blocks do not mix columns.
+  constexpr bool AS_IT_LIES = B2N && LOW;
+  // DIT passes at bit 0 without a short round end with a row's 16 consecutive
+  // words in each thread.  Stored straight from there, a warp's 16-byte stores
+  // would each touch 32 lines (12-bit passes 11 % slower), so these go through
+  // the tile, whose next words meanwhile wait in registers.
+  constexpr bool STAGED = !B2N && LOW && K % 4 == 0;
+  uint64_t x[STAGED ? 16 : 1];
+  auto first = [&](uint32_t c0) {
+    if constexpr (STAGED) {
+      const uint64_t *src = elem_at<K, LC>(in + (uint64_t)c0 * p.stride_in, e_in, p.stride_in, step_bytes);
 #pragma unroll
-    for (uint32_t i = 0; i < 8; i++) {
-      const uint32_t e = 2 * (tid + THREADS * i);
-      const uint32_t col = c0 + (e >> (K + LC));
-      if (col < tg.col_end) {
-        const uint64_t *src = elem_at<K, LC>(in + (uint64_t)c0 * p.stride_in, e, p.stride_in, step_bytes);
-        uint8_t *dst = tile + addr_of<K, LC, B2N, 0>(e);
-        if (p.vec_in) {
-          cp_async16(dst, src);
-        } else {
-          cp_async8(dst, src);
-          cp_async8(dst + 8, src + 1);
+      for (uint32_t s = 0; s < 16; s++) {
+        const uint32_t es = elem_of_slot<K, LC, B2N, 0>(s);
+        x[s] = c0 + ((e_in | es) >> (K + LC)) < tg.col_end ? __ldcg(elem_at<K, LC>(src, es, p.stride_in, step_bytes)) : 0;
+      }
+    } else if constexpr (AS_IT_LIES) {
+#pragma unroll
+      for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t e = 2 * (tid + THREADS * i);
+        const uint32_t col = c0 + (e >> (K + LC));
+        if (col < tg.col_end) {
+          const uint64_t *src = elem_at<K, LC>(in + (uint64_t)c0 * p.stride_in, e, p.stride_in, step_bytes);
+          uint8_t *dst = tile + addr_of<K, LC, B2N, 0>(e);
+          if (p.vec_in) {
+            cp_async16(dst, src);
+          } else {
+            cp_async8(dst, src);
+            cp_async8(dst + 8, src + 1);
+          }
         }
+      }
+    } else {
+      const uint64_t *src = elem_at<K, LC>(in + (uint64_t)c0 * p.stride_in, e_in, p.stride_in, step_bytes);
+#pragma unroll
+      for (uint32_t s = 0; s < 16; s++) {
+        const uint32_t es = elem_of_slot<K, LC, B2N, 0>(s);
+        if (c0 + ((e_in | es) >> (K + LC)) < tg.col_end)
+          cp_async8(tile + xor_part(a_in, addr_of<K, LC, B2N, 0>(es)), elem_at<K, LC>(src, es, p.stride_in, step_bytes));
       }
     }
     cp_async_commit();
-  };
-  uint64_t x[16];
-  auto load = [&](uint32_t c0) {
-    const uint64_t *src = elem_at<K, LC>(in + (uint64_t)c0 * p.stride_in, e_in, p.stride_in, step_bytes);
-#pragma unroll
-    for (uint32_t s = 0; s < 16; s++) {
-      const uint32_t es = elem_of_slot<K, LC, B2N, 0>(s);
-      x[s] = c0 + ((e_in | es) >> (K + LC)) < tg.col_end ? __ldcg(elem_at<K, LC>(src, es, p.stride_in, step_bytes)) : 0;
-    }
-  };
-  auto first = [&] {
-    if constexpr (COPY_IN)
-      copy_in(tg.col_begin);
-    else
-      load(tg.col_begin);
   };
   // the first column's words: before the tables, whose set-up then hides their
   // latency, or after them when the predecessor may still be running
   if (!tables_first) {
     if (p.overlap) wait_previous();
-    first();
+    first(tg.col_begin);
   }
 
   {
@@ -299,64 +312,79 @@ __device__ __forceinline__ void pass_body_tc(const PassParams &p, uint32_t bx, u
   }
   if (tables_first) {
     wait_previous();
-    first();
+    first(tg.col_begin);
   }
 
 #pragma unroll 1
   for (uint32_t c0 = tg.col_begin; c0 < tg.col_end; c0 += G) {
-    if constexpr (COPY_IN) {
-      cp_async_wait<0>();
-    } else {
-      // the row's 16 words: chunks of two
+    if constexpr (STAGED) {
 #pragma unroll
-      for (int s = 0; s < 16; s += 2)
+      for (uint32_t s = 0; s < 16; s += 2)
         *reinterpret_cast<ulonglong2 *>(tile + xor_part(a_in, addr_of<K, LC, B2N, 0>(elem_of_slot<K, LC, B2N, 0>(s)))) =
             make_ulonglong2(x[s], x[s + 1]);
+    } else {
+      cp_async_wait<0>();
     }
     middle_rounds<K, LC, B2N, 0>(ctx, tile, pw, img_top, img_full, img_short);
     constexpr Layout ql = RS::make(B2N, LAST);
     multiply(ctx, smem_u32(tile), ql.V < 4 ? img_short : ql.B == K - 4 ? img_top : img_full);
     const bool more = c0 + G < tg.col_end;
-    if constexpr (COPY_OUT) {
+    if constexpr (STAGED) {
+      const uint32_t a_out = addr_of<K, LC, B2N, LAST>(e_out);
       uint64_t even = 0;
       outputs(ctx, [&](int o, uint64_t y) {
         if (p.canon_out) y = gl::canon(y);
+        const uint32_t ee = elem_of_slot<K, LC, B2N, LAST>((uint32_t)o & ~1u);
         if (o & 1)
-          *reinterpret_cast<ulonglong2 *>(tile + xor_part(a_out, addr_of<K, LC, B2N, LAST>(elem_of_slot<K, LC, B2N, LAST>((uint32_t)o - 1)))) =
-              make_ulonglong2(even, y);
+          *reinterpret_cast<ulonglong2 *>(tile + xor_part(a_out, addr_of<K, LC, B2N, LAST>(ee))) = make_ulonglong2(even, y);
         else
           even = y;
       });
-      if (more) load(c0 + G);
+      if (more) first(c0 + G);
       __syncthreads();
 #pragma unroll
       for (uint32_t i = 0; i < 8; i++) {
         const uint32_t e = 2 * (tid + THREADS * i);
         if (c0 + (e >> (K + LC)) >= tg.col_end) continue;
         const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(tile + addr_of<K, LC, B2N, LAST>(e));
-        uint64_t *dst = elem_at<K, LC>(out + (uint64_t)c0 * p.stride_out, e, p.stride_out, step_bytes);
+        uint64_t *d = elem_at<K, LC>(out + (uint64_t)c0 * p.stride_out, e, p.stride_out, step_bytes);
         if (p.vec_out) {
-          *reinterpret_cast<ulonglong2 *>(dst) = v;
+          *reinterpret_cast<ulonglong2 *>(d) = v;
         } else {
-          dst[0] = v.x;
-          dst[1] = v.y;
+          d[0] = v.x;
+          d[1] = v.y;
         }
       }
       __syncthreads(); // the tile is free
-    } else {
-      if constexpr (COPY_IN) {
-        if (more) copy_in(c0 + G); // the operands have been read
-      }
-      uint64_t *dst = elem_at<K, LC>(out + (uint64_t)c0 * p.stride_out, e_out, p.stride_out, step_bytes);
-      outputs(ctx, [&](int o, uint64_t y) {
-        const uint32_t eo = elem_of_slot<K, LC, B2N, LAST>((uint32_t)o);
-        if (p.canon_out) y = gl::canon(y);
-        if (c0 + ((e_out | eo) >> (K + LC)) < tg.col_end) __stcg(elem_at<K, LC>(dst, eo, p.stride_out, step_bytes), y);
-      });
-      if constexpr (!COPY_IN) {
-        if (more) load(c0 + G);
-      }
+      continue;
     }
+    if (more) first(c0 + G); // the operands have been read: the tile is free
+    // straight from registers: neighbouring threads write neighbouring addresses,
+    // or (DIT, bit 0, short last round) a thread its row's runs of 2^V words, 16
+    // bytes at a time (10-bit passes: 10 % faster than through the tile)
+    uint64_t *dst = elem_at<K, LC>(out + (uint64_t)c0 * p.stride_out, e_out, p.stride_out, step_bytes);
+    uint64_t even = 0;
+    outputs(ctx, [&](int o, uint64_t y) {
+      if (p.canon_out) y = gl::canon(y);
+      const uint32_t eo = elem_of_slot<K, LC, B2N, LAST>((uint32_t)o);
+      if constexpr (!B2N && LOW) {
+        if (!(o & 1)) {
+          even = y;
+          return;
+        }
+        const uint32_t ee = elem_of_slot<K, LC, B2N, LAST>((uint32_t)o - 1);
+        if (c0 + ((e_out | ee) >> (K + LC)) >= tg.col_end) return;
+        uint64_t *d = elem_at<K, LC>(dst, ee, p.stride_out, step_bytes);
+        if (p.vec_out) {
+          __stcg(reinterpret_cast<ulonglong2 *>(d), make_ulonglong2(even, y));
+        } else {
+          __stcg(d, even);
+          __stcg(d + 1, y);
+        }
+      } else {
+        if (c0 + ((e_out | eo) >> (K + LC)) < tg.col_end) __stcg(elem_at<K, LC>(dst, eo, p.stride_out, step_bytes), y);
+      }
+    });
   }
   cp_async_wait<0>();
 }

@@ -16,9 +16,10 @@
 // of shift butterflies is 42 instructions per element; folding eight digits is
 // 15, and the tensor pipe, idle otherwise, does the sums (8180 multiply-adds
 // per clock and SM measured for M = 128, N = 128, K = 32 instructions, 64
-// cycles each).  Measured on B200, register-resident rounds including the
-// multiplications by powers: 853 G butterflies/s for this form against 820 for
-// the butterfly network, 1560 against 980 for rounds that need no powers.
+// cycles each).  Measured on B200, register-resident rounds: 850 G butterflies/s
+// with the multiplications by powers (the butterfly network: 820) and 1560
+// where a round needs none, which is why the kernels put as many powers as they
+// can into the matrices.
 //
 // Layout of a tile (4096 elements, 12 index bits): 256 rows of 16 words in the
 // K-major 128-byte-swizzle layout that the MMA's shared-memory descriptors
