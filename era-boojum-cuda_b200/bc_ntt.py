@@ -47,6 +47,7 @@ _u32, _u64, _sz, _b, _vp = ctypes.c_uint32, ctypes.c_uint64, ctypes.c_size_t, ct
 SIGNATURES = {
     "bc_ntt_context_create": [_u32, _u32],
     "bc_ntt_context_destroy": [],
+    "bc_ntt_wait_status": [_vp],
     "bc_batch_ntt_internal": [_vp, _vp, _u32, _u32, _u64, _u64, _b, _b, _u32, _u32, _vp],
     "bc_batch_ntt_out_of_place": [_vp, _sz, _vp, _sz, _u32, _u32, _u64, _u64, _u64, _u64, _b, _b, _u32, _u32, _vp],
     "bc_batch_ntt_in_place": [_vp, _sz, _u32, _u32, _u64, _u64, _b, _b, _u32, _u32, _vp],
@@ -168,6 +169,13 @@ class Context:
         if self.live:
             _check(lib().bc_ntt_context_destroy(), "Context.destroy")
             self.live = False
+
+
+def wait_status() -> int:
+    """1 when a kernel's bounded wait for its tensor-core products ran out since the last call, else 0."""
+    st = ctypes.c_uint32(0)
+    _check(lib().bc_ntt_wait_status(ctypes.byref(st)), "bc_ntt_wait_status")
+    return st.value
 
 
 def batch_ntt_internal(inputs_ptr: int, outputs_ptr: int, log_n: int, num_ntts: int,

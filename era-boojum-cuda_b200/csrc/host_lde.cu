@@ -96,7 +96,7 @@ cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *ho
     CK(cudaEventRecord(ev_in[b], hp.s_in));
     // transform (dense coset-major layout inside the chunk buffer)
     CK(cudaStreamWaitEvent(hp.s_comp, ev_in[b], 0));
-    CK(lde_fused(pl, d_in, d_out, log_n, cols, n, n, (uint64_t)cols * n, log_blowup, hp.s_comp));
+    CK(lde_fused(fit_plan(pl, log_n, cols), d_in, d_out, log_n, cols, n, n, (uint64_t)cols * n, log_blowup, hp.s_comp));
     CK(cudaEventRecord(ev_comp[b], hp.s_comp));
     // copy out every coset block of the chunk
     CK(cudaStreamWaitEvent(hp.s_out, ev_comp[b], 0));

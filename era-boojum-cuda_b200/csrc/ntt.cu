@@ -257,6 +257,33 @@ Plan default_plan(uint32_t log_n) {
   return pl;
 }
 
+// A plan whose lowest window is below 12 bits tiles columns together on the
+// tensor cores (2^(12 - K) of them).  With fewer columns than fill such a tile
+// (tc_window_ok) that pass, and with it the fused top window, would run on the
+// other kernels: a two-pass split with the next larger low window that is
+// filled is taken instead, 12 bits at most (B200, 2 x 2^22 plain: 3 passes on
+// the other kernels against 2 here), else one bit more in the low window
+// (2^13: 4 + 9 bits instead of 5 + 8, 6 % faster on the other kernels).
+Plan fit_plan(const Plan &pl, uint32_t log_n, uint32_t cols) {
+  const int low = pl.pass[pl.npasses - 1].K;
+  if (pl.npasses < 2 || pl.pass[pl.npasses - 1].C != 1 || low < 8 || tc_window_ok(low, 0, cols, true, true)) return pl;
+  auto split = [&](int k) {
+    const int top = (int)log_n - k;
+    Plan q{};
+    q.npasses = 2;
+    q.pass[0] = {(uint8_t)top, (uint8_t)(top <= 9 ? 8 : 4)};
+    q.pass[1] = {(uint8_t)k, 1};
+    q.knobs = pl.knobs;
+    return q;
+  };
+  for (int k = low + 1; k <= 12; k++) {
+    const int top = (int)log_n - k;
+    if ((top == 4 || top == 5 || (top >= 8 && top <= 10)) && tc_window_ok(k, 0, cols, true, true)) return split(k);
+  }
+  const int top = pl.pass[0].K;
+  return pl.npasses == 2 && (top == 5 || top == 9) && low < 12 ? split(low + 1) : pl;
+}
+
 static bool shape_supported(int K, int C) {
   if (C == 1) return K >= 1 && K <= 12;
   if (C == 8) return K >= 1 && K <= 9;
@@ -513,13 +540,23 @@ extern "C" cudaError_t bc_ntt_context_create(uint32_t powers_of_w_coarse_log_cou
 
 extern "C" cudaError_t bc_ntt_context_destroy(void) { return context_destroy_current(); }
 
+extern "C" cudaError_t bc_ntt_wait_status(uint32_t *status) {
+  const DevTables *t = device_tables();
+  if (!status) return cudaErrorInvalidValue;
+  if (!t) return cudaErrorInitializationError;
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = cudaMemcpy(status, t->wait_error, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && *status) e = cudaMemset(t->wait_error, 0, sizeof(uint32_t));
+  return e;
+}
+
 extern "C" cudaError_t bc_batch_ntt_internal(const uint64_t *inputs, uint64_t *outputs, uint32_t log_n,
                                              uint32_t num_ntts, uint64_t stride_in, uint64_t stride_out,
                                              bool bitrev_inputs, bool inverse, uint32_t log_extension_degree,
                                              uint32_t coset_index, cudaStream_t stream) {
   if (!ntt_args_ok(log_n, stride_in, stride_out, log_extension_degree, coset_index)) return cudaErrorInvalidValue;
   if (num_ntts && (!inputs || !outputs)) return cudaErrorInvalidValue;
-  return launch_ntt(tuned_plan(log_n, 0), inputs, outputs, log_n, num_ntts, stride_in, stride_out, bitrev_inputs,
+  return launch_ntt(fit_plan(tuned_plan(log_n, 0), log_n, num_ntts), inputs, outputs, log_n, num_ntts, stride_in, stride_out, bitrev_inputs,
                     inverse, log_extension_degree, coset_index, stream);
 }
 

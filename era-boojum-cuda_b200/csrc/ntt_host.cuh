@@ -70,6 +70,8 @@ Plan default_plan(uint32_t log_n);
 // The autotuned plan of the current device for an LDE (log_blowup >= 1) or a
 // plain NTT (log_blowup = 0), else default_plan (tune.cu).
 Plan tuned_plan(uint32_t log_n, uint32_t log_blowup);
+// The plan, or one with a larger low window for few columns.
+Plan fit_plan(const Plan &pl, uint32_t log_n, uint32_t cols);
 bool plan_valid(const Plan &pl, uint32_t log_n);
 
 // Scaling by base^i, i the natural index, spread over the passes: the index is

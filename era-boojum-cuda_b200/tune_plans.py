@@ -3,7 +3,7 @@
 
     python era-boojum-cuda_b200/tune_plans.py [--out era-boojum-cuda_b200/plans_b200.txt]
 
-For every log_n in 12..23 and blowup in {1 (plain NTT), 2, 4, 8} it times all
+For every log_n in 12..24 and blowup in {1 (plain NTT), 2, 4, 8} it times all
 candidate window splits and then the launch knobs of the best one (bc_autotune)
 on 2^27 input elements of columns (2^28 output elements at most) and keeps the
 fastest; bc_ntt.load_tuned_plans() loads the file into a process.
@@ -23,7 +23,7 @@ def main():
 
     ap = argparse.ArgumentParser()
     ap.add_argument("--out", default=os.path.join(HERE, "plans_b200.txt"))
-    ap.add_argument("--log-n", type=int, nargs=2, default=(12, 23))
+    ap.add_argument("--log-n", type=int, nargs=2, default=(12, 24))
     ap.add_argument("--reps", type=int, default=3)
     args = ap.parse_args()
     torch.cuda.set_device(0)

@@ -38,6 +38,13 @@ cudaError_t bc_ntt_context_create(uint32_t powers_of_w_coarse_log_count, uint32_
 /* Replaces Context::destroy (src/context.rs:284-296) for the current device. */
 cudaError_t bc_ntt_context_destroy(void);
 
+/* Whether a kernel's bounded wait for its tensor-core products has run out on
+ * the current device since the last call (then 1, and the results of that
+ * launch are invalid; else 0).  Such a kernel ends, with its tensor memory
+ * freed, instead of waiting for good; none has been seen to.  Synchronises
+ * with the device and clears the flag. */
+cudaError_t bc_ntt_wait_status(uint32_t *status);
+
 /* Replaces batch_ntt_internal (src/ntt.rs:179-191).
  * num_ntts columns of n = 2^log_n elements.
  *   bitrev_inputs = false: natural-order input, bit-reversed output

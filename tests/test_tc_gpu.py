@@ -120,3 +120,27 @@ def test_chains_in_a_graph_and_on_two_streams(gpu_ctx):
         g.replay()
     torch.cuda.synchronize()
     assert np.array_equal(to_host(a), want)
+    assert bc_ntt.wait_status() == 0
+
+
+@pytest.mark.parametrize("log_n,log_b", [(13, 1), (13, 2), (14, 1), (15, 3), (18, 1)])
+def test_few_columns_with_tuned_plans(gpu_ctx, log_n, log_b):
+    """Column counts on both sides of a low window's full tiles, where the plan in use changes."""
+    import torch
+
+    import bc_ntt
+    import oracle
+
+    old = bc_ntt.plan_table_export()
+    try:
+        assert bc_ntt.load_tuned_plans()
+        for cols in (1, 2, 3, 5, 6, 11, 12, 17) if log_n < 16 else (1, 3, 4):
+            n = 1 << log_n
+            x = raw_u64(np.random.default_rng(100 * log_n + cols), cols * n)
+            d, o = to_dev(x), torch.zeros(cols * n << log_b, dtype=torch.int64, device="cuda")
+            bc_ntt.lde(d, o, log_n, cols, log_b)
+            assert np.array_equal(to_host(o), oracle.lde(x, log_n, cols, n, log_b)), cols
+    finally:
+        bc_ntt.plan_table_clear()
+        if old:
+            bc_ntt.plan_table_import(old)
