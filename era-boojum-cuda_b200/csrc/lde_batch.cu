@@ -60,6 +60,12 @@ __host__ __device__ constexpr uint64_t make_item(uint32_t rec, uint32_t by, uint
 }
 
 constexpr uint32_t BATCH_THREADS = 256;
+// What the launch bounds, BATCH_SMEM_BYTES and the tensor memory (256 of 512
+// columns each) allow.  Not asked of the occupancy calculator: for kernels that
+// allocate tensor memory it answers 1 whatever their share (192 small jobs:
+// 2336 us with one CTA an SM, 1447 with two).  The schedule needs no particular number: items
+// are taken in order by CTAs that run.
+constexpr int BATCH_CTAS_PER_SM = 2;
 // largest bodies: the top window of 12 bits with one forward table, and the
 // tensor-core top window of 10 bits (two CTAs an SM either way)
 constexpr uint32_t BATCH_SMEM_BYTES = TOP_RESIDENT_SMEM_MAX > tc::top_tc_smem_bytes<10, true>()
@@ -301,7 +307,7 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
     if (jb.num_cols && (!jb.evals_bitrev || !jb.out)) return cudaErrorInvalidValue;
     if (standalone_min_ctas && standalone && jb.num_cols) {
       std::vector<LdeStep> own;
-      if (!build_lde_steps(tuned_plan(jb.log_n, jb.log_blowup), jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols,
+      if (!build_lde_steps(fit_plan(tuned_plan(jb.log_n, jb.log_blowup), jb.log_n, jb.num_cols), jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols,
                            jb.stride_in, jb.stride_out, jb.coset_stride, jb.log_blowup, false, 8, 8, own))
         return cudaErrorInvalidConfiguration;
       uint64_t min_ctas = ~0ull;
@@ -325,7 +331,7 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
           return false;
       return true;
     };
-    if (!build(tuned_plan(jb.log_n, jb.log_blowup)) && !build(default_plan(jb.log_n)))
+    if (!build(fit_plan(tuned_plan(jb.log_n, jb.log_blowup), jb.log_n, jb.num_cols)) && !build(default_plan(jb.log_n)))
       return cudaErrorInvalidConfiguration;
     max_depth = std::max(max_depth, steps[j].size());
   }
@@ -398,13 +404,7 @@ extern "C" cudaError_t bc_lde_batch_plan_create_ex(const bc_lde_job *jobs, uint3
     return e;                                                                                                          \
   }
   CK(cudaFuncSetAttribute(lde_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_SMEM_BYTES));
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lde_batch_kernel, BATCH_THREADS, BATCH_SMEM_BYTES));
-  if (per_sm < 1) {
-    free_plan(p);
-    return cudaErrorInvalidConfiguration;
-  }
-  p->grid = (uint32_t)(per_sm * sm_count());
+  p->grid = (uint32_t)(BATCH_CTAS_PER_SM * sm_count());
   if (p->n_records) {
     CK(cudaMalloc(&p->d_records, recs.size() * sizeof(BatchRecord)));
     CK(cudaMemcpy(p->d_records, recs.data(), recs.size() * sizeof(BatchRecord), cudaMemcpyHostToDevice));
@@ -529,11 +529,7 @@ cudaError_t noalloc_setup(int dev, void **base, int *grid) {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(lde_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lde_batch_kernel, BATCH_THREADS, BATCH_SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    g_noalloc_grid[dev] = per_sm * sm_count();
+    g_noalloc_grid[dev] = BATCH_CTAS_PER_SM * sm_count();
     g_noalloc_base[dev] = p;
   }
   *base = g_noalloc_base[dev];
@@ -581,11 +577,7 @@ cudaError_t batch_enqueue_into(const bc_lde_job *jobs, uint32_t n_jobs, void *de
   if (!grid) {
     e = cudaFuncSetAttribute(lde_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lde_batch_kernel, BATCH_THREADS, BATCH_SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    grid = per_sm * sm_count();
+    grid = BATCH_CTAS_PER_SM * sm_count();
     if (dev >= 0 && dev < 64) grid_cache[dev].store(grid, std::memory_order_relaxed);
   }
   unsigned char *d = static_cast<unsigned char *>(dev_scratch);
