@@ -55,6 +55,7 @@ SIGNATURES = {
     "bc_autotune": [_u32, _u32, _u32, _u32, _vp, _sz],
     "bc_plan_table_export": [_vp, _sz, _vp],
     "bc_plan_table_import": [ctypes.c_char_p],
+    "bc_plan_table_import_defaults": [ctypes.c_char_p],
     "bc_plan_table_clear": [],
     "bc_lde_plain": [_vp, _vp, _u32, _u32, _u64, _u64, _u64, _u32, _vp],
     "bc_lde_fused": [_vp, _vp, _u32, _u32, _u64, _u64, _u64, _u32, _vp],
@@ -405,11 +406,15 @@ PLANS_PATH = os.path.join(_HERE, "plans_b200.txt")
 
 
 def load_tuned_plans(path: str = PLANS_PATH) -> bool:
-    """Loads a plan table written by tune_plans.py (the current device must have a context)."""
+    """Loads a plan table written by tune_plans.py (the current device must have a context): the shipped one as
+    default entries, another one as the caller's own plans."""
     if not os.path.exists(path):
         return False
     text = "".join(line for line in open(path) if line.strip() and not line.startswith("#"))
-    plan_table_import(text)
+    if path == PLANS_PATH:
+        _check(lib().bc_plan_table_import_defaults(text.encode()), "bc_plan_table_import_defaults")
+    else:
+        plan_table_import(text)
     return True
 
 

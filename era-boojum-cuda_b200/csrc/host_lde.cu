@@ -72,7 +72,6 @@ cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *ho
                              cudaStream_t caller) {
   const uint64_t n = 1ull << log_n, nb = 1ull << log_blowup;
   const uint64_t in_words = (uint64_t)chunk * n, out_words = in_words * nb;
-  const Plan pl = tuned_plan(log_n, log_blowup);
   cudaError_t e;
 #define CK(x)                                                                                                          \
   if ((e = (x)) != cudaSuccess) return e;
@@ -96,7 +95,8 @@ cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *ho
     CK(cudaEventRecord(ev_in[b], hp.s_in));
     // transform (dense coset-major layout inside the chunk buffer)
     CK(cudaStreamWaitEvent(hp.s_comp, ev_in[b], 0));
-    CK(lde_fused(fit_plan(pl, log_n, cols), d_in, d_out, log_n, cols, n, n, (uint64_t)cols * n, log_blowup, hp.s_comp));
+    CK(lde_fused(call_plan(log_n, log_blowup, cols), d_in, d_out, log_n, cols, n, n, (uint64_t)cols * n, log_blowup,
+                 hp.s_comp));
     CK(cudaEventRecord(ev_comp[b], hp.s_comp));
     // copy out every coset block of the chunk
     CK(cudaStreamWaitEvent(hp.s_out, ev_comp[b], 0));

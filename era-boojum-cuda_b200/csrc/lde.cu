@@ -372,8 +372,8 @@ extern "C" cudaError_t bc_lde_fused(const uint64_t *evals_bitrev, uint64_t *out,
                                     uint32_t log_blowup, cudaStream_t stream) {
   if (!lde_args_ok(log_n, num_cols, stride_in, stride_out, coset_stride, log_blowup)) return cudaErrorInvalidValue;
   if (num_cols && (!evals_bitrev || !out)) return cudaErrorInvalidValue;
-  return lde_fused(fit_plan(tuned_plan(log_n, log_blowup), log_n, num_cols), evals_bitrev, out, log_n, num_cols, stride_in, stride_out, coset_stride,
-                   log_blowup, stream);
+  return lde_fused(call_plan(log_n, log_blowup, num_cols), evals_bitrev, out, log_n, num_cols, stride_in, stride_out,
+                   coset_stride, log_blowup, stream);
 }
 
 extern "C" cudaError_t bc_lde_fused_profiled(const uint64_t *evals_bitrev, uint64_t *out, uint32_t log_n,
@@ -382,7 +382,7 @@ extern "C" cudaError_t bc_lde_fused_profiled(const uint64_t *evals_bitrev, uint6
                                              cudaEvent_t *events, uint32_t num_events, uint32_t *num_kernels) {
   if (!lde_args_ok(log_n, num_cols, stride_in, stride_out, coset_stride, log_blowup)) return cudaErrorInvalidValue;
   if (num_cols && (!evals_bitrev || !out)) return cudaErrorInvalidValue;
-  const Plan pl = fit_plan(tuned_plan(log_n, log_blowup), log_n, num_cols);
+  const Plan pl = call_plan(log_n, log_blowup, num_cols);
   if (num_kernels) *num_kernels = (uint32_t)(2 * pl.npasses - 1);
   return lde_fused(pl, evals_bitrev, out, log_n, num_cols, stride_in, stride_out, coset_stride, log_blowup, stream,
                    events, num_events);

@@ -307,8 +307,8 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
     if (jb.num_cols && (!jb.evals_bitrev || !jb.out)) return cudaErrorInvalidValue;
     if (standalone_min_ctas && standalone && jb.num_cols) {
       std::vector<LdeStep> own;
-      if (!build_lde_steps(fit_plan(tuned_plan(jb.log_n, jb.log_blowup), jb.log_n, jb.num_cols), jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols,
-                           jb.stride_in, jb.stride_out, jb.coset_stride, jb.log_blowup, false, 8, 8, own))
+      if (!build_lde_steps(call_plan(jb.log_n, jb.log_blowup, jb.num_cols), jb.evals_bitrev, jb.out, jb.log_n,
+                           jb.num_cols, jb.stride_in, jb.stride_out, jb.coset_stride, jb.log_blowup, false, 8, 8, own))
         return cudaErrorInvalidConfiguration;
       uint64_t min_ctas = ~0ull;
       for (const LdeStep &st : own) min_ctas = std::min<uint64_t>(min_ctas, (uint64_t)st.grid.x * st.grid.y);
@@ -317,7 +317,7 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
         continue; // steps[j] stays empty: no records for this job
       }
     }
-    // the tuned plan, or the built-in one when the tuned plan uses a window shape this kernel does not carry
+    // the call's plan, or the built-in one when that uses a window shape this kernel does not carry
     auto build = [&](const Plan &pl) {
       if (!build_lde_steps(pl, jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols, jb.stride_in, jb.stride_out,
                            jb.coset_stride, jb.log_blowup, true, 16, 16, steps[j]))
@@ -331,7 +331,7 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
           return false;
       return true;
     };
-    if (!build(fit_plan(tuned_plan(jb.log_n, jb.log_blowup), jb.log_n, jb.num_cols)) && !build(default_plan(jb.log_n)))
+    if (!build(call_plan(jb.log_n, jb.log_blowup, jb.num_cols)) && !build(default_plan(jb.log_n)))
       return cudaErrorInvalidConfiguration;
     max_depth = std::max(max_depth, steps[j].size());
   }

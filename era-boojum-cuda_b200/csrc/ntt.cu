@@ -266,6 +266,7 @@ Plan default_plan(uint32_t log_n) {
 // (2^13: 4 + 9 bits instead of 5 + 8, 6 % faster on the other kernels).
 Plan fit_plan(const Plan &pl, uint32_t log_n, uint32_t cols) {
   const int low = pl.pass[pl.npasses - 1].K;
+  if (cols > 65535) return pl; // the tensor-core kernels' limit, not few
   if (pl.npasses < 2 || pl.pass[pl.npasses - 1].C != 1 || low < 8 || tc_window_ok(low, 0, cols, true, true)) return pl;
   auto split = [&](int k) {
     const int top = (int)log_n - k;
@@ -556,8 +557,8 @@ extern "C" cudaError_t bc_batch_ntt_internal(const uint64_t *inputs, uint64_t *o
                                              uint32_t coset_index, cudaStream_t stream) {
   if (!ntt_args_ok(log_n, stride_in, stride_out, log_extension_degree, coset_index)) return cudaErrorInvalidValue;
   if (num_ntts && (!inputs || !outputs)) return cudaErrorInvalidValue;
-  return launch_ntt(fit_plan(tuned_plan(log_n, 0), log_n, num_ntts), inputs, outputs, log_n, num_ntts, stride_in, stride_out, bitrev_inputs,
-                    inverse, log_extension_degree, coset_index, stream);
+  return launch_ntt(call_plan(log_n, 0, num_ntts), inputs, outputs, log_n, num_ntts, stride_in, stride_out,
+                    bitrev_inputs, inverse, log_extension_degree, coset_index, stream);
 }
 
 extern "C" cudaError_t bc_batch_ntt_out_of_place(const uint64_t *inputs_matrix, size_t inputs_len,

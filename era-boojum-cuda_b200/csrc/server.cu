@@ -312,8 +312,8 @@ void launch_device_group(bc_lde_server *s, std::vector<Request *> group, bool ba
   } else {
     const Request &r = *group[0];
     const uint64_t n = 1ull << r.log_n;
-    e = lde_fused(fit_plan(tuned_plan(r.log_n, r.log_blowup), r.log_n, r.cols), r.in, r.out, r.log_n, r.cols, n, n, (uint64_t)r.cols * n,
-                  r.log_blowup, s->s_dev);
+    e = lde_fused(call_plan(r.log_n, r.log_blowup, r.cols), r.in, r.out, r.log_n, r.cols, n, n,
+                  (uint64_t)r.cols * n, r.log_blowup, s->s_dev);
   }
   GroupCtx *g = nullptr;
   cudaEvent_t done = nullptr;

@@ -10,9 +10,14 @@
 // smallest top window), then tunes the plan's launch knobs (ntt_host.cuh
 // Knobs: column walks, top-window table mode and double-buffering, pass
 // occupancy) one at a time on that window split, keeping a value only when it
-// is more than 1 % faster; LDE and NTT entry points consult the table and fall back to the built-in
-// plan.  Candidates use only window shapes that
-// every kernel (the persistent batch kernel included) can run.
+// is more than 1 % faster; LDE and NTT entry points consult the table and fall
+// back to the built-in plan.  Candidates use only window shapes that every
+// kernel (the persistent batch kernel included) can run.
+//
+// Entries are of two kinds.  What the caller imported or autotuned is run as it
+// is, whatever the columns.  Default entries (bc_plan_table_import_defaults:
+// the shipped table) stand in for built-in plans and, like these, are fitted
+// to calls of few columns (fit_plan).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,7 +36,11 @@ namespace bc {
 
 namespace {
 constexpr int TUNE_MAX_DEVICES = 64;
-std::map<uint32_t, Plan> g_table[TUNE_MAX_DEVICES];
+struct Entry {
+  Plan plan;
+  bool fit; // a default entry
+};
+std::map<uint32_t, Entry> g_table[TUNE_MAX_DEVICES];
 std::mutex g_table_mutex;
 
 uint32_t key(uint32_t log_n, uint32_t log_blowup) { return (log_blowup << 8) | log_n; }
@@ -113,15 +122,15 @@ const KnobAxis KNOB_AXES[] = {
 };
 } // namespace
 
-// The plan of an LDE (log_blowup >= 1) or of a plain NTT (log_blowup = 0).
-Plan tuned_plan(uint32_t log_n, uint32_t log_blowup) {
+Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols) {
+  Entry en{default_plan(log_n), true};
   const int d = current_device();
   if (d >= 0 && d < TUNE_MAX_DEVICES) {
     std::lock_guard<std::mutex> lock(g_table_mutex);
     auto it = g_table[d].find(key(log_n, log_blowup));
-    if (it != g_table[d].end()) return it->second;
+    if (it != g_table[d].end()) en = it->second;
   }
-  return default_plan(log_n);
+  return en.fit ? fit_plan(en.plan, log_n, cols) : en.plan;
 }
 
 } // namespace bc
@@ -234,7 +243,7 @@ extern "C" cudaError_t bc_autotune(uint32_t log_n, uint32_t log_blowup, uint32_t
   if (e != cudaSuccess) return e;
   {
     std::lock_guard<std::mutex> lock(g_table_mutex);
-    g_table[dev][key(log_n, log_blowup)] = best;
+    g_table[dev][key(log_n, log_blowup)] = Entry{best, false};
   }
   rep += "best " + plan_str(best) + "\n";
   if (report && report_len) {
@@ -254,10 +263,10 @@ extern "C" cudaError_t bc_plan_table_export(char *buf, size_t len, size_t *neede
     std::lock_guard<std::mutex> lock(g_table_mutex);
     for (auto &kv : g_table[dev]) {
       char line[128];
-      int w = snprintf(line, sizeof line, "%u %u %d", kv.first & 0xFF, kv.first >> 8, kv.second.npasses);
-      for (int i = 0; i < kv.second.npasses; i++)
-        w += snprintf(line + w, sizeof line - w, " %d %d", kv.second.pass[i].K, kv.second.pass[i].C);
-      const Knobs &k = kv.second.knobs;
+      const Plan &pl = kv.second.plan;
+      int w = snprintf(line, sizeof line, "%u %u %d", kv.first & 0xFF, kv.first >> 8, pl.npasses);
+      for (int i = 0; i < pl.npasses; i++) w += snprintf(line + w, sizeof line - w, " %d %d", pl.pass[i].K, pl.pass[i].C);
+      const Knobs &k = pl.knobs;
       if (k.walk || k.top_walk || k.top_mode || k.top_dbuf || k.occ)
         snprintf(line + w, sizeof line - w, " k %d %d %d %d %d", k.walk, k.top_walk, k.top_mode, k.top_dbuf, k.occ);
       t += line;
@@ -272,7 +281,7 @@ extern "C" cudaError_t bc_plan_table_export(char *buf, size_t len, size_t *neede
   return cudaSuccess;
 }
 
-extern "C" cudaError_t bc_plan_table_import(const char *text) {
+static cudaError_t import_table(const char *text, bool fit) {
   if (!text) return cudaErrorInvalidValue;
   const int dev = current_device();
   if (dev < 0 || dev >= TUNE_MAX_DEVICES) return cudaErrorInvalidDevice;
@@ -308,9 +317,12 @@ extern "C" cudaError_t bc_plan_table_import(const char *text) {
     while (*p == ' ' || *p == '\n' || *p == '\r' || *p == '\t') p++;
   }
   std::lock_guard<std::mutex> lock(g_table_mutex);
-  for (auto &kv : parsed) g_table[dev][kv.first] = kv.second;
+  for (auto &kv : parsed) g_table[dev][kv.first] = Entry{kv.second, fit};
   return cudaSuccess;
 }
+
+extern "C" cudaError_t bc_plan_table_import(const char *text) { return import_table(text, false); }
+extern "C" cudaError_t bc_plan_table_import_defaults(const char *text) { return import_table(text, true); }
 
 extern "C" cudaError_t bc_plan_table_clear(void) {
   const int dev = current_device();

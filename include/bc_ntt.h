@@ -93,7 +93,10 @@ cudaError_t bc_batch_ntt_with_plan(const uint64_t *inputs, uint64_t *outputs, ui
  * the fused LDE -- how many stages its middle kernel fuses (the top window).
  * Each device keeps a table keyed by (log_n, log_blowup), log_blowup = 0 for
  * the plain NTT; every entry point here uses the table's plan when present and
- * the built-in one otherwise.  bc_autotune times every candidate plan on the
+ * the built-in one otherwise.  A plan that the caller imported or autotuned runs
+ * as it is, whatever the columns; built-in plans, and those imported as
+ * defaults, may be replaced by one with a larger low window for calls with too
+ * few columns to fill theirs.  bc_autotune times every candidate plan on the
  * current device (num_cols columns, reps timed runs after one warm-up; it
  * allocates and frees its own scratch and synchronises), then the launch knobs
  * of the fastest window split one at a time (column-group walk of the pass and
@@ -109,6 +112,11 @@ cudaError_t bc_autotune(uint32_t log_n, uint32_t log_blowup, uint32_t num_cols, 
  * 3 recomputed tables; top_dbuf 1 off, 2 on; occ 2 or 3 CTAs per SM). */
 cudaError_t bc_plan_table_export(char *buf, size_t len, size_t *needed);
 cudaError_t bc_plan_table_import(const char *text);
+/* The same text as default entries, which take the place of built-in plans
+ * (the shipped plans_b200.txt without its comment lines).  Export does not tell
+ * the two kinds apart: what it wrote comes back through bc_plan_table_import as
+ * the caller's own. */
+cudaError_t bc_plan_table_import_defaults(const char *text);
 cudaError_t bc_plan_table_clear(void);
 
 /* ---- coset low-degree extension ------------------------------------------

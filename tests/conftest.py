@@ -51,3 +51,32 @@ def gpu_ctx():
     ctx = bc_ntt.Context.create(12, 12)
     yield ctx
     torch.cuda.synchronize()
+
+
+def kernel_names(fn):
+    """Kernels that fn() launches, in no particular order, as "name<template arguments>" (booleans as 0 / 1): read
+    from a graph that fn() is captured into, so nothing runs."""
+    import re
+
+    import torch
+    from cuda.bindings import driver
+
+    def ok(res):
+        assert res[0] == driver.CUresult.CUDA_SUCCESS, res[0]
+        return res[1] if len(res) == 2 else res[1:]
+
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    graph = driver.CUgraph(g.raw_cuda_graph())
+    _, count = ok(driver.cuGraphGetNodes(graph))
+    nodes, _ = ok(driver.cuGraphGetNodes(graph, count))
+    names = []
+    for n in nodes:
+        if ok(driver.cuGraphNodeGetType(n)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = ok(driver.cuGraphKernelNodeGetParams(n))
+        name = ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern)).decode()
+        m = re.search(r"\d([a-z_]+)I((?:L[bij]\d+E)+)E", name)
+        names.append(f"{m[1]}<{','.join(re.findall(r'L[bij](\d+)E', m[2]))}>" if m else name)
+    return names

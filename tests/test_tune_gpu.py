@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 import oracle
-from conftest import raw_u64, to_dev, to_host
+from conftest import kernel_names, raw_u64, to_dev, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -98,3 +98,41 @@ def test_plan_knobs_validation(gpu_ctx):
         with pytest.raises(ValueError):
             bc_ntt.plan_table_import(bad)
     bc_ntt.plan_table_clear()
+
+
+def test_callers_plans_run_as_they_are(gpu_ctx):
+    """An imported or autotuned plan is used as it is, also for columns that do not fill its low window's tiles; only
+    built-in plans and default entries may be fitted to the columns."""
+    import bc_ntt
+    import torch
+
+    d = torch.zeros(16 << 13, dtype=torch.int64, device="cuda")
+    out = torch.zeros(32 << 13, dtype=torch.int64, device="cuda")
+
+    def windows(cols):
+        """Window bits of the kernels of a fused LDE and of a plain transform."""
+        lde = kernel_names(lambda: bc_ntt.lde(d, out, 13, cols, 1))
+        ntt = kernel_names(lambda: bc_ntt.batch_ntt_internal(d.data_ptr(), out.data_ptr(), 13, cols, 1 << 13, 1 << 13,
+                                                             False, False, 0, 0))
+        return sorted(int(k.split("<")[1].split(",")[0]) for k in lde), sorted(
+            int(k.split("<")[1].split(",")[0].rstrip(">")) for k in ntt)
+
+    text = "13 0 2 5 8 8 1\n13 1 2 5 8 8 1\n"
+    try:
+        bc_ntt.plan_table_clear()
+        bc_ntt.plan_table_import(text)
+        for cols in (1, 5, 11, 16):  # 16 columns fill an 8-bit window's tile
+            assert windows(cols) == ([5, 8, 8], [5, 8]), cols
+        assert bc_ntt.plan_table_export() == text
+        bc_ntt._check(bc_ntt.lib().bc_plan_table_import_defaults(text.encode()), "import_defaults")
+        assert bc_ntt.plan_table_export() == text
+        assert windows(16) == ([5, 8, 8], [5, 8])
+        assert windows(11)[0] == [4, 9, 9]
+        bc_ntt.autotune(13, 1, 5, reps=1)  # an entry measured at its column count replaces the default
+        line = [x for x in bc_ntt.plan_table_export().splitlines() if x.startswith("13 1")][0].split()
+        top, low = int(line[3]), int(line[5])
+        assert windows(5)[0] == sorted([top, low, low])
+        with pytest.raises(ValueError):
+            bc_ntt._check(bc_ntt.lib().bc_plan_table_import_defaults(b"13 1 2 5 8 9 1\n"), "import_defaults")
+    finally:
+        bc_ntt.plan_table_clear()
