@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <climits>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -43,15 +44,36 @@ __host__ __device__ constexpr uint32_t shape_id(bool top, bool b2n, int K, int C
          (C == 1 ? 0u : C == 2 ? 1u : C == 4 ? 2u : 3u);
 }
 
+// A record holds a kernel's parameters up to their tables, which are the same
+// for all of them (two thirds of a record otherwise, and the schedules that
+// live in fixed arrays would hold that many fewer jobs).  They end at
+// PARAM_BYTES whichever kind they are, so that a CTA can keep the tables behind
+// them in shared memory and copy only the record from item to item.
+constexpr size_t PASS_PARAM_BYTES = offsetof(PassParams, tabs), TOP_PARAM_BYTES = offsetof(LdeTopParams, tabs);
+constexpr size_t PARAM_BYTES = PASS_PARAM_BYTES > TOP_PARAM_BYTES ? PASS_PARAM_BYTES : TOP_PARAM_BYTES;
+static_assert(PASS_PARAM_BYTES + sizeof(DevTables) == sizeof(PassParams) &&
+                  TOP_PARAM_BYTES + sizeof(DevTables) == sizeof(LdeTopParams) && PASS_PARAM_BYTES % 8 == 0 &&
+                  TOP_PARAM_BYTES % 8 == 0,
+              "the tables come last");
 struct BatchRecord {
   uint32_t shape;
   int32_t pred;     // record that must be complete before any item of this one, or -1
   uint32_t n_items; // CTAs of this kernel
   uint32_t tc;      // a tensor-core body: shape is a tc_shape_id
-  union {
-    PassParams pass;
-    LdeTopParams top;
-  } u;
+  alignas(8) unsigned char params[PARAM_BYTES];
+};
+static_assert(sizeof(BatchRecord) == 16 + PARAM_BYTES, "no gap before the tables");
+
+// The record of the item a CTA works on, the tables behind it.
+struct ItemRecord {
+  BatchRecord rec;
+  DevTables tabs;
+  __device__ const PassParams &pass() const {
+    return *reinterpret_cast<const PassParams *>(rec.params + PARAM_BYTES - PASS_PARAM_BYTES);
+  }
+  __device__ const LdeTopParams &top() const {
+    return *reinterpret_cast<const LdeTopParams *>(rec.params + PARAM_BYTES - TOP_PARAM_BYTES);
+  }
 };
 
 // item = record (16 bits) | column chunk by (20 bits) | tile position bx (28 bits)
@@ -93,15 +115,15 @@ bool batch_shape_supported(uint32_t id) {
 }
 
 template <bool TOP, bool B2N, int K, int C>
-__device__ __noinline__ void run_shape(const BatchRecord &rec, uint32_t bx, uint32_t by, uint64_t *smem) {
+__device__ __noinline__ void run_shape(const ItemRecord &rec, uint32_t bx, uint32_t by, uint64_t *smem) {
   if constexpr (TOP)
-    top_body<K, C>(rec.u.top, bx, by, smem);
+    top_body<K, C>(rec.top(), bx, by, smem);
   else
-    pass_body<K, C, B2N, B2N>(rec.u.pass, bx, by, smem); // LDE passes: b2n ones are the inverse transform
+    pass_body<K, C, B2N, B2N>(rec.pass(), bx, by, smem); // LDE passes: b2n ones are the inverse transform
 }
 
-__device__ __forceinline__ void run_body(const BatchRecord &rec, uint32_t bx, uint32_t by, uint64_t *smem) {
-  switch (rec.shape) {
+__device__ __forceinline__ void run_body(const ItemRecord &rec, uint32_t bx, uint32_t by, uint64_t *smem) {
+  switch (rec.rec.shape) {
 #define BC_CASE(TOP, B2N, K, C)                                                                                      \
   case shape_id(TOP, B2N, K, C):                                                                                     \
     run_shape<TOP, B2N, K, C>(rec, bx, by, smem);                                                                    \
@@ -137,17 +159,17 @@ bool batch_tc_shape_supported(uint32_t id) {
 }
 
 template <int K, bool WIDE>
-__device__ __noinline__ void run_tc_top(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
-  tc::top_body_tc<K, WIDE>(rec.u.top, bx, by, smem, ctx, false);
+__device__ __noinline__ void run_tc_top(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
+  tc::top_body_tc<K, WIDE>(rec.top(), bx, by, smem, ctx, false);
 }
 template <bool B2N, bool LOW, int K>
-__device__ __noinline__ void run_tc_pass(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
-  tc::pass_body_tc<K, LOW, B2N, B2N>(rec.u.pass, bx, by, smem, ctx, false);
+__device__ __noinline__ void run_tc_pass(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
+  tc::pass_body_tc<K, LOW, B2N, B2N>(rec.pass(), bx, by, smem, ctx, false);
 }
 
-__device__ __forceinline__ void run_tc_body(const BatchRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem,
+__device__ __forceinline__ void run_tc_body(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem,
                                             tc::Ctx &ctx) {
-  switch (rec.shape) {
+  switch (rec.rec.shape) {
 #define BC_CASE(K, WIDE)                                                                                             \
   case tc_shape_id(true, false, false, K):                                                                           \
     run_tc_top<K, WIDE>(rec, bx, by, smem, ctx);                                                                     \
@@ -173,14 +195,18 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 
 // status bit 0: a dependency wait expired, bit 1: a tensor-core completion wait did (the batch's results are invalid).
 // wait_limit: SM clock cycles one dependency wait may take (read once per CTA).
+// tabs: the tables of every record.
 __global__ void __launch_bounds__(BATCH_THREADS, 2)
     lde_batch_kernel(const BatchRecord *__restrict__ recs, const uint64_t *__restrict__ items, uint32_t n_items,
-                     uint32_t *done, uint32_t *next, uint32_t *status, const long long *wait_limit) {
+                     uint32_t *done, uint32_t *next, uint32_t *status, const long long *wait_limit,
+                     const DevTables *__restrict__ tabs) {
   extern __shared__ uint64_t smem[];
   __shared__ uint32_t s_idx, s_ok;
-  __shared__ BatchRecord s_rec; // the item's kernel parameters, read by the body from shared memory
+  __shared__ ItemRecord s_rec; // the item's kernel parameters, read by the body from shared memory
   __shared__ __align__(16) uint64_t s_tc[2]; // barrier and tensor-memory address of the tensor-core bodies
   const long long timeout_cycles = threadIdx.x == 0 ? *wait_limit : 0;
+  for (uint32_t w = threadIdx.x; w < sizeof(DevTables) / 4; w += blockDim.x)
+    reinterpret_cast<uint32_t *>(&s_rec.tabs)[w] = reinterpret_cast<const uint32_t *>(tabs)[w];
   tc::Ctx ctx = tc::begin(s_tc);
   uint8_t *const tc_smem = reinterpret_cast<uint8_t *>(smem) + ((1024 - (tc::smem_u32(smem) & 1023)) & 1023);
   for (;;) {
@@ -193,7 +219,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
     const BatchRecord &rec = recs[r];
     static_assert(sizeof(BatchRecord) % 4 == 0, "record copy by words");
     for (uint32_t w = threadIdx.x; w < sizeof(BatchRecord) / 4; w += blockDim.x)
-      reinterpret_cast<uint32_t *>(&s_rec)[w] = reinterpret_cast<const uint32_t *>(&rec)[w];
+      reinterpret_cast<uint32_t *>(&s_rec.rec)[w] = reinterpret_cast<const uint32_t *>(&rec)[w];
     if (threadIdx.x == 0) {
       uint32_t ok = 1;
       if (rec.pred >= 0) {
@@ -212,7 +238,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
     }
     __syncthreads();
     if (s_ok) {
-      if (s_rec.tc)
+      if (s_rec.rec.tc)
         run_tc_body(s_rec, bx, by, tc_smem, ctx);
       else
         run_body(s_rec, bx, by, smem);
@@ -365,9 +391,9 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
       r.pred = last[j];
       r.n_items = st.grid.x * st.grid.y;
       if (st.top)
-        r.u.top = st.topp;
+        std::memcpy(r.params + PARAM_BYTES - TOP_PARAM_BYTES, &st.topp, TOP_PARAM_BYTES);
       else
-        r.u.pass = st.pass;
+        std::memcpy(r.params + PARAM_BYTES - PASS_PARAM_BYTES, &st.pass, PASS_PARAM_BYTES);
       const uint32_t rid = (uint32_t)recs.size();
       if (rid >= (1u << 16)) return cudaErrorInvalidConfiguration;
       recs.push_back(r);
@@ -435,7 +461,7 @@ extern "C" cudaError_t bc_lde_batch_plan_create_ex(const bc_lde_job *jobs, uint3
     if (ec == cudaSuccess && p->n_items) {
       lde_batch_kernel<<<p->grid, BATCH_THREADS, BATCH_SMEM_BYTES, cs>>>(
           p->d_records, p->d_items, p->n_items, p->d_counters, p->d_counters + p->n_records,
-          p->d_counters + p->n_records + 1, wait_limit_slot(p->d_counters, p->n_records));
+          p->d_counters + p->n_records + 1, wait_limit_slot(p->d_counters, p->n_records), device_tables_on_gpu());
       ec = cudaGetLastError();
     }
     if (ec == cudaSuccess && !standalone.empty()) ec = cudaStreamWaitEvent(cs, join, 0);
@@ -585,7 +611,7 @@ cudaError_t batch_enqueue_into(const bc_lde_job *jobs, uint32_t n_jobs, void *de
   lde_batch_kernel<<<grid, BATCH_THREADS, BATCH_SMEM_BYTES, stream>>>(
       reinterpret_cast<const BatchRecord *>(d + counters_bytes),
       reinterpret_cast<const uint64_t *>(d + counters_bytes + recs_bytes), (uint32_t)items.size(), counters,
-      counters + n_rec, counters + n_rec + 1, wait_limit_slot(counters, n_rec));
+      counters + n_rec, counters + n_rec + 1, wait_limit_slot(counters, n_rec), device_tables_on_gpu());
   return cudaGetLastError();
 }
 } // namespace bc
@@ -635,7 +661,8 @@ extern "C" cudaError_t bc_lde_batch_noalloc(const bc_lde_job *jobs, uint32_t n_j
     lde_batch_kernel<<<grid, BATCH_THREADS, BATCH_SMEM_BYTES, stream>>>(d_recs, d_items, (uint32_t)items.size(),
                                                                          counters, counters + n_rec,
                                                                          counters + n_rec + 1,
-                                                                         wait_limit_slot(counters, n_rec));
+                                                                         wait_limit_slot(counters, n_rec),
+                                                                         device_tables_on_gpu());
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

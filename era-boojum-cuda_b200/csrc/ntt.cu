@@ -42,12 +42,14 @@ inline uint32_t brev(uint32_t x, unsigned bits) {
 // ---------------------------------------------------------------- context
 namespace {
 constexpr int MAX_DEVICES = 64;
+constexpr size_t TC_TAIL_TABS = 16; // offset of the copy of the tables behind the matrices; the error word before it
+
 struct DeviceCtx {
   bool live = false;
   uint64_t *block = nullptr;
   uint64_t *top_pw = nullptr; // precomputed top-window power tables
   uint64_t *top_pw_st = nullptr; // the same for the short-round-on-top partition
-  uint8_t *tc = nullptr; // tensor-core matrices, then the wait-error word
+  uint8_t *tc = nullptr; // tensor-core matrices, then the wait-error word and a copy of tabs
   DevTables tabs{};
   int sms = 0;
 };
@@ -107,6 +109,11 @@ const DevTables *device_tables() {
   const int d = current_device();
   if (d < 0 || d >= MAX_DEVICES || !g_ctx[d].live) return nullptr;
   return &g_ctx[d].tabs;
+}
+
+const DevTables *device_tables_on_gpu() {
+  const DevTables *t = device_tables();
+  return t ? reinterpret_cast<const DevTables *>(t->tc_img + tc_table_bytes() + TC_TAIL_TABS) : nullptr;
 }
 
 int sm_count() {
@@ -179,11 +186,13 @@ cudaError_t context_create_current() {
   if (e == cudaSuccess) e = cudaMalloc(&c.top_pw_st, top_pw_words() * sizeof(uint64_t));
   if (e == cudaSuccess) e = top_pw_fill<1, 0>(c.tabs, c.top_pw);
   if (e == cudaSuccess) e = top_pw_fill<1, 1>(c.tabs, c.top_pw_st);
-  if (e == cudaSuccess) e = cudaMalloc(&c.tc, tc_table_bytes() + 16);
-  if (e == cudaSuccess) e = cudaMemset(c.tc + tc_table_bytes(), 0, 16);
+  if (e == cudaSuccess) e = cudaMalloc(&c.tc, tc_table_bytes() + TC_TAIL_TABS + sizeof(DevTables));
+  if (e == cudaSuccess) e = cudaMemset(c.tc + tc_table_bytes(), 0, TC_TAIL_TABS);
   if (e == cudaSuccess) e = tc_fill_tables(c.tc, c.tabs);
   c.tabs.tc_img = c.tc;
   c.tabs.wait_error = reinterpret_cast<uint32_t *>(c.tc + tc_table_bytes());
+  if (e == cudaSuccess)
+    e = cudaMemcpy(c.tc + tc_table_bytes() + TC_TAIL_TABS, &c.tabs, sizeof(DevTables), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     cudaFree(c.block);

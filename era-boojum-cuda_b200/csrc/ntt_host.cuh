@@ -53,6 +53,7 @@ struct Plan {
 // Per-device tables; returns nullptr when the context was not created on the
 // current device.
 const DevTables *device_tables();
+const DevTables *device_tables_on_gpu(); // a copy of them in device memory
 
 // Power tables (ntt_pass.cuh) of top windows, precomputed per device: for each
 // K <= 12 the inverse table of H = 0, and for each log_blowup b with

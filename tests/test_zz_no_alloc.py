@@ -105,3 +105,26 @@ def test_noalloc_batch_rejects_stream_capture(gpu_ctx):
     del graph
     _run_noalloc(arr, 1)
     _check_against_fused(jobs)
+
+
+@pytest.mark.parametrize("log_n,cols,jobs_per_batch", [(8, 1, 36000), (13, 1, 7400)])
+def test_noalloc_batch_holds_many_small_jobs(gpu_ctx, log_n, cols, jobs_per_batch):
+    """The fixed array holds 36,000 one-kernel or 7,400 three-kernel jobs: 16 bytes and a kernel's own parameters for
+    each kernel, 8 bytes a work item."""
+    import torch
+
+    import bc_ntt
+
+    n, log_b = 1 << log_n, 1
+    (job,), _ = _jobs(np.random.default_rng(3), [(log_n, cols, log_b)])
+    outs = torch.full((jobs_per_batch, (cols * n) << log_b), 0x11, dtype=torch.int64, device="cuda")
+    arr = (bc_ntt.LdeJob * jobs_per_batch)()
+    for i in range(jobs_per_batch):
+        arr[i] = bc_ntt.LdeJob(job[0].data_ptr(), outs.data_ptr() + 8 * i * outs.shape[1], n, n, cols * n, log_n, cols, log_b, 0)
+    status = ctypes.c_uint32(0xFFFF)
+    rc = bc_ntt.lib().bc_lde_batch_noalloc(ctypes.cast(arr, ctypes.c_void_p), jobs_per_batch,
+                                           torch.cuda.current_stream().cuda_stream, ctypes.byref(status))
+    assert rc == 0 and status.value == 0
+    ref = torch.empty_like(job[1])
+    bc_ntt.lde(job[0], ref, log_n, cols, log_b)
+    assert bool((outs == ref).all())
