@@ -48,6 +48,7 @@ SIGNATURES = {
     "bc_ntt_context_create": [_u32, _u32],
     "bc_ntt_context_destroy": [],
     "bc_ntt_wait_status": [_vp],
+    "bc_ntt_set_wait_limit": [_u32],
     "bc_batch_ntt_internal": [_vp, _vp, _u32, _u32, _u64, _u64, _b, _b, _u32, _u32, _vp],
     "bc_batch_ntt_out_of_place": [_vp, _sz, _vp, _sz, _u32, _u32, _u64, _u64, _u64, _u64, _b, _b, _u32, _u32, _vp],
     "bc_batch_ntt_in_place": [_vp, _sz, _u32, _u32, _u64, _u64, _b, _b, _u32, _u32, _vp],
@@ -177,6 +178,11 @@ def wait_status() -> int:
     st = ctypes.c_uint32(0)
     _check(lib().bc_ntt_wait_status(ctypes.byref(st)), "bc_ntt_wait_status")
     return st.value
+
+
+def set_wait_limit(tries: int = 1 << 20):
+    """Bound of those waits, in tries of about 4 microseconds; 0: every one runs out at once."""
+    _check(lib().bc_ntt_set_wait_limit(tries), "bc_ntt_set_wait_limit")
 
 
 def batch_ntt_internal(inputs_ptr: int, outputs_ptr: int, log_n: int, num_ntts: int,

@@ -160,11 +160,15 @@ bool batch_tc_shape_supported(uint32_t id) {
 
 template <int K, bool WIDE>
 __device__ __noinline__ void run_tc_top(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
-  tc::top_body_tc<K, WIDE>(rec.top(), bx, by, smem, ctx, false);
+  tc::Ctx c = ctx; // in registers
+  tc::top_body_tc<K, WIDE>(rec.top(), bx, by, smem, c, false);
+  ctx = c;
 }
 template <bool B2N, bool LOW, int K>
 __device__ __noinline__ void run_tc_pass(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem, tc::Ctx &ctx) {
-  tc::pass_body_tc<K, LOW, B2N, B2N>(rec.pass(), bx, by, smem, ctx, false);
+  tc::Ctx c = ctx;
+  tc::pass_body_tc<K, LOW, B2N, B2N>(rec.pass(), bx, by, smem, c, false);
+  ctx = c;
 }
 
 __device__ __forceinline__ void run_tc_body(const ItemRecord &rec, uint32_t bx, uint32_t by, uint8_t *smem,
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
   const long long timeout_cycles = threadIdx.x == 0 ? *wait_limit : 0;
   for (uint32_t w = threadIdx.x; w < sizeof(DevTables) / 4; w += blockDim.x)
     reinterpret_cast<uint32_t *>(&s_rec.tabs)[w] = reinterpret_cast<const uint32_t *>(tabs)[w];
-  tc::Ctx ctx = tc::begin(s_tc);
+  tc::Ctx ctx = tc::begin(s_tc, tabs->wait_tries);
   uint8_t *const tc_smem = reinterpret_cast<uint8_t *>(smem) + ((1024 - (tc::smem_u32(smem) & 1023)) & 1023);
   for (;;) {
     if (threadIdx.x == 0) s_idx = atomicAdd(next, 1u);

@@ -147,11 +147,7 @@ template <bool WIDE> __device__ __forceinline__ void top_multiply(Ctx &c, uint32
   if constexpr (!WIDE) {
     multiply(c, tile, img);
   } else {
-    fence_smem_to_mma();
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
-    if (threadIdx.x == 0 && !c.bad) {
+    products(c, [&] {
 #pragma unroll
       for (uint32_t k = 0; k < 8; k++) {
         const uint64_t a = operand_desc(tile + (k >> 2) * (TILE_BYTES / 2)) + 2 * (k & 3);
@@ -164,13 +160,7 @@ template <bool WIDE> __device__ __forceinline__ void top_multiply(Ctx &c, uint32
                      "l"(a), "l"(b), "r"(MMA_DESC_WIDE), "r"(k)
                      : "memory");
       }
-      mma_commit(c.bar);
-    }
-    __syncwarp();
-    if (!c.bad) c.bad = !mbar_wait(c.bar, c.phase);
-    c.phase ^= 1;
-    __syncwarp();
-    fence_after_sync();
+    });
   }
 }
 
@@ -373,7 +363,7 @@ template <int K, bool WIDE> __global__ void __launch_bounds__(THREADS, 2) top_ke
   uint8_t *smem = tc_smem + ((1024 - (smem_u32(tc_smem) & 1023)) & 1023);
   uint64_t *slot = reinterpret_cast<uint64_t *>(smem + TILE_BYTES + top_tc_images<K, WIDE>()) +
                    ((top_tc_pw_words<K, WIDE>() + 1) & ~1u);
-  Ctx ctx = begin(slot);
+  Ctx ctx = begin(slot, p.tabs.wait_tries);
   allow_next(); // with its tensor memory in hand: no CTA of this launch can wait for one of the next
   top_body_tc<K, WIDE>(p, blockIdx.x, blockIdx.y, smem, ctx, in_first_wave(p.overlap));
   end(ctx, p.tabs.wait_error);

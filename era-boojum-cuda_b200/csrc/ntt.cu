@@ -12,6 +12,7 @@
 #include "../../include/bc_ntt.h"
 #include "ntt_host.cuh"
 #include "ntt_pass.cuh"
+#include "tc.cuh"
 
 namespace bc {
 
@@ -191,6 +192,7 @@ cudaError_t context_create_current() {
   if (e == cudaSuccess) e = tc_fill_tables(c.tc, c.tabs);
   c.tabs.tc_img = c.tc;
   c.tabs.wait_error = reinterpret_cast<uint32_t *>(c.tc + tc_table_bytes());
+  c.tabs.wait_tries = tc::WAIT_TRIES;
   if (e == cudaSuccess)
     e = cudaMemcpy(c.tc + tc_table_bytes() + TC_TAIL_TABS, &c.tabs, sizeof(DevTables), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -558,6 +560,15 @@ extern "C" cudaError_t bc_ntt_wait_status(uint32_t *status) {
   if (e == cudaSuccess) e = cudaMemcpy(status, t->wait_error, sizeof(uint32_t), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && *status) e = cudaMemset(t->wait_error, 0, sizeof(uint32_t));
   return e;
+}
+
+extern "C" cudaError_t bc_ntt_set_wait_limit(uint32_t tries) {
+  DevTables *t = const_cast<DevTables *>(device_tables());
+  if (!t) return cudaErrorInitializationError;
+  cudaError_t e = cudaDeviceSynchronize(); // runs already enqueued finish with the old limit
+  if (e != cudaSuccess) return e;
+  t->wait_tries = tries > tc::WAIT_TRIES ? tc::WAIT_TRIES : tries;
+  return cudaMemcpy(const_cast<DevTables *>(device_tables_on_gpu()), t, sizeof(DevTables), cudaMemcpyHostToDevice);
 }
 
 extern "C" cudaError_t bc_batch_ntt_internal(const uint64_t *inputs, uint64_t *outputs, uint32_t log_n,

@@ -28,17 +28,24 @@ template <int K> __host__ __device__ constexpr uint32_t pass_smem_bytes() {
   return 1024 + TILE_BYTES + pass_images<K>() * IMG_BYTES + PowerTable<K>::words * 8 + 32;
 }
 
+// A thread whose wait ran out waits for nothing more and goes on to the end:
+// what it then reads and overwrites early is its own CTA's tile and
+// accumulators, so the launch's results are invalid (and reported) but nothing
+// else is touched.  The issuing thread also issues nothing more.  Telling the
+// whole CTA at its next barrier instead cost 1 to 5 % of every kernel.
 struct Ctx {
   uint32_t bar, tmem, phase;
-  bool bad; // a wait ran out: nothing more is issued or waited for
+  uint32_t tries; // bound of a wait
+  uint32_t bad;   // 0, or 1 + the barrier's phase whose wait ran out
 };
 
 // Barrier and tensor memory of a CTA; ends with a barrier.  slot: 16 bytes of shared memory.
-__device__ __forceinline__ Ctx begin(uint64_t *slot) {
+__device__ __forceinline__ Ctx begin(uint64_t *slot, uint32_t tries) {
   Ctx c;
   c.bar = smem_u32(slot);
   c.phase = 0;
-  c.bad = false;
+  c.tries = tries;
+  c.bad = 0;
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot + 1)),
                  "r"(TMEM_COLS)
@@ -56,8 +63,14 @@ __device__ __forceinline__ Ctx begin(uint64_t *slot) {
   return c;
 }
 
+// Frees the tensor memory.  Products that the issuing thread gave up on may
+// still be running: it waits for them once more first, so that they do not end
+// in the memory of whoever is given it next.
 __device__ __forceinline__ void end(const Ctx &c, uint32_t *error) {
-  if (c.bad && error) atomicExch(error, 1u);
+  if (c.bad) {
+    if (threadIdx.x == 0) mbar_wait(c.bar, c.bad - 1, WAIT_TRIES);
+    if (error) *(volatile uint32_t *)error = 1u;
+  }
   fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32)
@@ -68,25 +81,32 @@ __device__ __forceinline__ void end(const Ctx &c, uint32_t *error) {
 // overlap): only those can start before the predecessor has ended.
 __device__ __forceinline__ bool in_first_wave(uint32_t wave) { return blockIdx.y * gridDim.x + blockIdx.x < wave; }
 
-// The tile times the matrix at img; orders this CTA's shared-memory stores
-// before, and returns when every operand has been read and all sums are in
-// tensor memory.
-__device__ __forceinline__ void multiply(Ctx &c, uint32_t tile, uint32_t img) {
+// One round's products, issued by one thread: orders this CTA's shared-memory
+// stores before, and returns when every operand has been read and all sums are
+// in tensor memory (or, c.bad, without).
+template <class F> __device__ __forceinline__ void products(Ctx &c, F &&issue) {
   fence_smem_to_mma();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   if (threadIdx.x == 0 && !c.bad) {
-    const uint64_t b = operand_desc(img);
-    mma_128x128(c.tmem, operand_desc(tile), b);
-    mma_128x128(c.tmem + 128, operand_desc(tile + TILE_BYTES / 2), b);
+    issue();
     mma_commit(c.bar);
   }
   __syncwarp();
-  if (!c.bad) c.bad = !mbar_wait(c.bar, c.phase);
+  if (!c.bad && !mbar_wait(c.bar, c.phase, c.tries)) c.bad = 1 + c.phase;
   c.phase ^= 1;
   __syncwarp();
   fence_after_sync();
+}
+
+// The tile times the matrix at img.
+__device__ __forceinline__ void multiply(Ctx &c, uint32_t tile, uint32_t img) {
+  products(c, [&] {
+    const uint64_t b = operand_desc(img);
+    mma_128x128(c.tmem, operand_desc(tile), b);
+    mma_128x128(c.tmem + 128, operand_desc(tile + TILE_BYTES / 2), b);
+  });
 }
 
 // use(o, y) for the 16 outputs of the thread's row, the reads of four outputs
@@ -394,7 +414,7 @@ template <int K, bool LOW, bool B2N, bool INV> __global__ void __launch_bounds__
   extern __shared__ __align__(1024) uint8_t tc_smem[];
   uint8_t *smem = tc_smem + ((1024 - (smem_u32(tc_smem) & 1023)) & 1023);
   uint64_t *slot = reinterpret_cast<uint64_t *>(smem + TILE_BYTES + pass_images<K>() * IMG_BYTES) + ((PowerTable<K>::words + 1) & ~1u);
-  Ctx ctx = begin(slot);
+  Ctx ctx = begin(slot, p.tabs.wait_tries);
   allow_next(); // with its tensor memory in hand: no CTA of this launch can wait for one of the next
   pass_body_tc<K, LOW, B2N, INV>(p, blockIdx.x, blockIdx.y, smem, ctx, in_first_wave(p.overlap));
   end(ctx, p.tabs.wait_error);

@@ -61,6 +61,8 @@ struct DevTables {
   uint64_t inv_pow2[TW_LOG + 1]; // 2^-k
   const uint8_t *tc_img; // matrices of the tensor-core rounds (tc.cuh, img_index)
   uint32_t *wait_error;  // set by a kernel whose bounded completion wait ran out
+  uint32_t wait_tries;   // that bound (tc.cuh, WAIT_TRIES)
+  uint32_t pad_;
 };
 
 } // namespace bc

@@ -43,7 +43,9 @@ constexpr uint32_t TILE_BYTES = TILE * 8;       // two M = 128 operands
 constexpr uint32_t THREADS = TILE / 16;         // one row a thread
 constexpr uint32_t IMG_BYTES = 16384;           // one B matrix, 128 x 128 bytes
 constexpr uint32_t TMEM_COLS = 256;             // accumulators: 2 x (128 lanes x 128 columns)
-constexpr uint32_t WAIT_TRIES = 1u << 22;       // bound of a completion wait (each try suspends for a while itself)
+// Bound of a completion wait, in tries: one suspends the thread for about 4 us
+// when nothing arrives (measured on B200, with or without a time hint), so 4 s.
+constexpr uint32_t WAIT_TRIES = 1u << 20;
 
 // ---------------------------------------------------------------- instructions
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -119,9 +121,9 @@ __device__ __forceinline__ void wait_ld(uint32_t (&r)[32]) {
                ::"memory");
 }
 
-// Waits for the completion of phase `parity`; false when the bound ran out.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < WAIT_TRIES; i++) {
+// Waits for the completion of phase `parity`; false when the tries ran out.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t tries) {
+  for (uint32_t i = 0; i < tries; i++) {
     uint32_t ok;
     asm volatile("{\n\t"
                  ".reg .pred p;\n\t"

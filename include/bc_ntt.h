@@ -39,11 +39,20 @@ cudaError_t bc_ntt_context_create(uint32_t powers_of_w_coarse_log_count, uint32_
 cudaError_t bc_ntt_context_destroy(void);
 
 /* Whether a kernel's bounded wait for its tensor-core products has run out on
- * the current device since the last call (then 1, and the results of that
- * launch are invalid; else 0).  Such a kernel ends, with its tensor memory
- * freed, instead of waiting for good; none has been seen to.  Synchronises
- * with the device and clears the flag. */
+ * the current device since the last call (then 1, and the results of the
+ * launches since then are suspect; else 0).  Such a kernel issues nothing more,
+ * waits once more, also bounded, for products in flight, frees its tensor
+ * memory and ends, instead of waiting for good; none has been seen to.  Should
+ * that second wait run out too, other launches on the device at that time are
+ * suspect as well.  Synchronises with the device and clears the flag, which is
+ * one for all callers on the device. */
 cudaError_t bc_ntt_wait_status(uint32_t *status);
+/* Sets that bound on the current device, in tries of about 4 microseconds
+ * (default and largest value: 2^20, about 4 s).  With 0 every such wait runs
+ * out at once, which is how a program tests what it does then.  Waits for the
+ * device first; launches enqueued later use it, captured graphs (but for batch
+ * plans) keep theirs.  Not to be called while another thread launches. */
+cudaError_t bc_ntt_set_wait_limit(uint32_t tries);
 
 /* Replaces batch_ntt_internal (src/ntt.rs:179-191).
  * num_ntts columns of n = 2^log_n elements.

@@ -144,3 +144,44 @@ def test_few_columns_with_tuned_plans(gpu_ctx, log_n, log_b):
         bc_ntt.plan_table_clear()
         if old:
             bc_ntt.plan_table_import(old)
+
+
+@pytest.mark.parametrize("log_n,cols,log_b,plan", [(12, 9, 0, "1 12 1"), (16, 9, 0, "2 8 8 8 1"), (14, 17, 1, "2 4 8 10 1"),
+                                                   (16, 9, 3, "2 5 8 11 1"), (20, 5, 1, "3 4 8 8 8 8 1"),
+                                                   (17, 16, 2, "2 8 8 9 1"), (22, 2, 1, "2 10 4 12 1")])
+def test_waits_that_run_out_are_reported(gpu_ctx, log_n, cols, log_b, plan):
+    """With a limit of no tries every wait for products runs out at once: the kernels end, say so, and hand their
+    tensor memory on only when their products are done; with the default again, the next results are exact."""
+    import torch
+
+    import bc_ntt
+
+    n = 1 << log_n
+    x = to_dev(raw_u64(np.random.default_rng(log_n), cols * n))
+    out, want = (torch.zeros(cols * n << log_b, dtype=torch.int64, device="cuda") for _ in range(2))
+
+    def run(o):
+        if log_b:
+            bc_ntt.lde(x, o, log_n, cols, log_b)
+        else:
+            bc_ntt.batch_ntt_internal(x.data_ptr(), o.data_ptr(), log_n, cols, n, n, True, True, 0, 0)
+
+    old = bc_ntt.plan_table_export()
+    try:
+        bc_ntt.plan_table_import(f"{log_n} {log_b} {plan}\n")
+        run(want)
+        assert bc_ntt.wait_status() == 0
+        bc_ntt.set_wait_limit(0)
+        for _ in range(3):
+            run(out)
+        assert bc_ntt.wait_status() == 1
+        assert bc_ntt.wait_status() == 0
+        bc_ntt.set_wait_limit()
+        run(out)
+        assert bc_ntt.wait_status() == 0
+        assert torch.equal(out, want)
+    finally:
+        bc_ntt.set_wait_limit()
+        bc_ntt.plan_table_clear()
+        if old:
+            bc_ntt.plan_table_import(old)
