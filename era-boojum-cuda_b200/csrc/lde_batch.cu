@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
     }
   }
   if (ctx.bad) atomicOr(status, 2u);
-  tc::end(ctx, nullptr);
+  tc::end(ctx, s_rec.tabs.wait_error);
 }
 
 } // namespace bc

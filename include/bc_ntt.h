@@ -190,9 +190,10 @@ cudaError_t bc_lde_host(const uint64_t *host_evals_bitrev, uint64_t *host_out, u
  * as needed (the job buffers are bound at plan time).  Plan creation
  * allocates the schedule on the current device (records, items, counters:
  * about 8 bytes per CTA-sized work item) and synchronises; bc_lde_batch_run
- * is asynchronous on the stream.  The kernel's dependency waits are bounded
- * (about 4 s each); bc_lde_batch_status returns status bit 0 if one expired,
- * in which case that run's outputs are invalid. */
+ * is asynchronous on the stream.  The kernel's waits are bounded (about 4 s
+ * each): bc_lde_batch_status returns status bit 0 if one for a dependency ran
+ * out, bit 1 if one for tensor-core products did (bc_ntt_wait_status then
+ * returns 1 too); with either, that run's outputs are invalid. */
 typedef struct bc_lde_job {
   const uint64_t *evals_bitrev;
   uint64_t *out;
@@ -241,8 +242,9 @@ cudaError_t bc_lde_batch_plan_destroy(bc_lde_batch_plan *plan);
  * whose work overlaps on the GPU (different streams, not ordered by events)
  * race and corrupt each other; calls ordered on one stream are safe.
  * status (optional): if non-null, the call waits for the stream and stores
- * the batch status word (bit 0: a bounded dependency wait expired and the
- * outputs are invalid). */
+ * the batch status word (bits 0 and 1 as for bc_lde_batch_status; with either,
+ * the outputs are invalid).  Without it, a wait for products that ran out
+ * still shows in bc_ntt_wait_status. */
 cudaError_t bc_lde_batch_noalloc(const bc_lde_job *jobs, uint32_t n_jobs, cudaStream_t stream, uint32_t *status);
 
 /* ---- the integer ceiling of the transform arithmetic ------------------------

@@ -167,3 +167,38 @@ def test_batch_wait_limit_expires_then_recovers(gpu_ctx):
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
     plan.close()
+
+
+def test_batch_reports_product_waits_that_run_out(gpu_ctx):
+    """With a limit of no tries the batch kernel's waits for products run out: status bit 1, and the device's flag
+    also when nobody reads the batch's status; with the default again, the next run is exact."""
+    import ctypes
+
+    import bc_ntt
+    import torch
+
+    jobs = _mixed_jobs(np.random.default_rng(100), [(14, 17, 1), (16, 9, 2), (11, 5, 1)])
+    plan = bc_ntt.LdeBatch([j[:5] for j in jobs])
+    arr = (bc_ntt.LdeJob * len(jobs))()
+    for i, (ev, out, log_n, cols, log_b, _) in enumerate(jobs):
+        n = 1 << log_n
+        arr[i] = bc_ntt.LdeJob(ev.data_ptr(), out.data_ptr(), n, n, cols * n, log_n, cols, log_b, 0)
+    assert bc_ntt.wait_status() == 0
+    try:
+        bc_ntt.set_wait_limit(0)
+        plan.run()
+        assert plan.status() == 2
+        assert bc_ntt.wait_status() == 1
+        rc = bc_ntt.lib().bc_lde_batch_noalloc(ctypes.cast(arr, ctypes.c_void_p), len(jobs),
+                                               torch.cuda.current_stream().cuda_stream, None)
+        assert rc == 0
+        assert bc_ntt.wait_status() == 1
+    finally:
+        bc_ntt.set_wait_limit()
+    plan.run()
+    assert plan.status() == 0 and bc_ntt.wait_status() == 0
+    for ev, out, log_n, cols, log_b, _ in jobs:
+        ref = torch.empty_like(out)
+        bc_ntt.lde(ev, ref, log_n, cols, log_b)
+        assert torch.equal(out, ref)
+    plan.close()
