@@ -69,7 +69,7 @@ uint32_t host_chunk_cols(uint32_t log_n, uint32_t num_cols, uint32_t log_blowup,
 cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *host_out, uint32_t log_n,
                              uint32_t num_cols, uint64_t stride_in, uint64_t stride_out, uint64_t coset_stride,
                              uint32_t log_blowup, uint64_t *workspace, uint32_t chunk, bool caller_ordered,
-                             cudaStream_t caller) {
+                             cudaStream_t caller, uint32_t *failed) {
   const uint64_t n = 1ull << log_n, nb = 1ull << log_blowup;
   const uint64_t in_words = (uint64_t)chunk * n, out_words = in_words * nb;
   cudaError_t e;
@@ -96,7 +96,7 @@ cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *ho
     // transform (dense coset-major layout inside the chunk buffer)
     CK(cudaStreamWaitEvent(hp.s_comp, ev_in[b], 0));
     CK(lde_fused(call_plan(log_n, log_blowup, cols), d_in, d_out, log_n, cols, n, n, (uint64_t)cols * n, log_blowup,
-                 hp.s_comp));
+                 hp.s_comp, nullptr, 0, failed));
     CK(cudaEventRecord(ev_comp[b], hp.s_comp));
     // copy out every coset block of the chunk
     CK(cudaStreamWaitEvent(hp.s_out, ev_comp[b], 0));

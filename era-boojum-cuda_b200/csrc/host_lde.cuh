@@ -29,10 +29,11 @@ uint32_t host_chunk_cols(uint32_t log_n, uint32_t num_cols, uint32_t log_blowup,
 // Enqueues a whole host LDE on the pipe's streams.  With `caller_ordered`,
 // the work starts after what is already queued on `caller` and `caller` waits
 // for its end (stream 0, the legacy default stream, is a valid caller);
-// without it, the end is the pipe's copy-out stream.
+// without it, the end is the pipe's copy-out stream.  failed (optional): a word
+// that is set when a bounded wait of a kernel ran out (lde_fused).
 cudaError_t host_lde_enqueue(HostPipe &hp, const uint64_t *host_in, uint64_t *host_out, uint32_t log_n,
                              uint32_t num_cols, uint64_t stride_in, uint64_t stride_out, uint64_t coset_stride,
                              uint32_t log_blowup, uint64_t *workspace, uint32_t chunk, bool caller_ordered,
-                             cudaStream_t caller);
+                             cudaStream_t caller, uint32_t *failed = nullptr);
 
 } // namespace bc

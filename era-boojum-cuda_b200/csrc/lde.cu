@@ -331,7 +331,7 @@ cudaError_t launch_lde_step(const LdeStep &st, cudaStream_t stream) {
 
 cudaError_t lde_fused(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_cols,
                       uint64_t stride_in, uint64_t stride_out, uint64_t coset_stride, uint32_t log_blowup,
-                      cudaStream_t stream, cudaEvent_t *ev, uint32_t n_ev) {
+                      cudaStream_t stream, cudaEvent_t *ev, uint32_t n_ev, uint32_t *failed) {
   if (!device_tables()) return cudaErrorInitializationError;
   if (num_cols == 0) return cudaSuccess;
   std::vector<LdeStep> steps;
@@ -340,7 +340,8 @@ cudaError_t lde_fused(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_
     return cudaErrorInvalidConfiguration;
   uint32_t ev_used = 0;
   if (ev_used < n_ev) cudaEventRecord(ev[ev_used++], stream);
-  for (const LdeStep &st : steps) {
+  for (LdeStep &st : steps) {
+    if (failed) st.pass.tabs.wait_error = st.topp.tabs.wait_error = failed;
     cudaError_t e = launch_lde_step(st, stream);
     if (e != cudaSuccess) return e;
     if (ev_used < n_ev) cudaEventRecord(ev[ev_used++], stream);

@@ -672,14 +672,17 @@ cudaError_t launch_lde_step(const LdeStep &st, cudaStream_t stream);
 
 // Enqueues a batch of LDE jobs (bc_lde_job, include/bc_ntt.h) as one
 // persistent launch with its schedule in caller-owned device scratch, staged
-// through caller-owned pinned memory (lde_batch.cu).
+// through caller-owned pinned memory (lde_batch.cu).  failed (optional): a word
+// that is set when a bounded wait of either kind ran out, in place of the
+// device's flag for waits for products.
 cudaError_t batch_enqueue_into(const bc_lde_job *jobs, uint32_t n_jobs, void *dev_scratch, void *host_staging,
-                               size_t scratch_bytes, cudaStream_t stream);
+                               size_t scratch_bytes, cudaStream_t stream, uint32_t *failed = nullptr);
 
 // Launches the fused LDE's kernels on `stream`; events (optional): ev[0] is
-// recorded before the first kernel and ev[j + 1] after kernel j.
+// recorded before the first kernel and ev[j + 1] after kernel j; failed
+// (optional): as for batch_enqueue_into.
 cudaError_t lde_fused(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_cols,
                       uint64_t stride_in, uint64_t stride_out, uint64_t coset_stride, uint32_t log_blowup,
-                      cudaStream_t stream, cudaEvent_t *ev = nullptr, uint32_t n_ev = 0);
+                      cudaStream_t stream, cudaEvent_t *ev = nullptr, uint32_t n_ev = 0, uint32_t *failed = nullptr);
 
 } // namespace bc

@@ -199,11 +199,12 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 
 // status bit 0: a dependency wait expired, bit 1: a tensor-core completion wait did (the batch's results are invalid).
 // wait_limit: SM clock cycles one dependency wait may take (read once per CTA).
-// tabs: the tables of every record.
+// tabs: the tables of every record.  failed: set with either bit, or null; bit 1
+// sets the device's flag otherwise.
 __global__ void __launch_bounds__(BATCH_THREADS, 2)
     lde_batch_kernel(const BatchRecord *__restrict__ recs, const uint64_t *__restrict__ items, uint32_t n_items,
                      uint32_t *done, uint32_t *next, uint32_t *status, const long long *wait_limit,
-                     const DevTables *__restrict__ tabs) {
+                     const DevTables *__restrict__ tabs, uint32_t *failed) {
   extern __shared__ uint64_t smem[];
   __shared__ uint32_t s_idx, s_ok;
   __shared__ ItemRecord s_rec; // the item's kernel parameters, read by the body from shared memory
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
           if (clock64() - t0 > timeout_cycles) {
             ok = 0;
             atomicOr(status, 1u);
+            if (failed) *(volatile uint32_t *)failed = 1u;
             break;
           }
           __nanosleep(128);
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2)
     }
   }
   if (ctx.bad) atomicOr(status, 2u);
-  tc::end(ctx, s_rec.tabs.wait_error);
+  tc::end(ctx, failed ? failed : s_rec.tabs.wait_error);
 }
 
 } // namespace bc
@@ -465,7 +467,8 @@ extern "C" cudaError_t bc_lde_batch_plan_create_ex(const bc_lde_job *jobs, uint3
     if (ec == cudaSuccess && p->n_items) {
       lde_batch_kernel<<<p->grid, BATCH_THREADS, BATCH_SMEM_BYTES, cs>>>(
           p->d_records, p->d_items, p->n_items, p->d_counters, p->d_counters + p->n_records,
-          p->d_counters + p->n_records + 1, wait_limit_slot(p->d_counters, p->n_records), device_tables_on_gpu());
+          p->d_counters + p->n_records + 1, wait_limit_slot(p->d_counters, p->n_records), device_tables_on_gpu(),
+          nullptr);
       ec = cudaGetLastError();
     }
     if (ec == cudaSuccess && !standalone.empty()) ec = cudaStreamWaitEvent(cs, join, 0);
@@ -578,7 +581,7 @@ namespace bc {
 // until the kernel has.  A batch whose schedule exceeds scratch_bytes returns
 // cudaErrorInvalidValue before anything is enqueued.
 cudaError_t batch_enqueue_into(const bc_lde_job *jobs, uint32_t n_jobs, void *dev_scratch, void *host_staging,
-                               size_t scratch_bytes, cudaStream_t stream) {
+                               size_t scratch_bytes, cudaStream_t stream, uint32_t *failed) {
   if (n_jobs && !jobs) return cudaErrorInvalidValue;
   if (!dev_scratch || !host_staging || (uintptr_t)dev_scratch % 256 || (uintptr_t)host_staging % 256)
     return cudaErrorInvalidValue;
@@ -615,7 +618,8 @@ cudaError_t batch_enqueue_into(const bc_lde_job *jobs, uint32_t n_jobs, void *de
   lde_batch_kernel<<<grid, BATCH_THREADS, BATCH_SMEM_BYTES, stream>>>(
       reinterpret_cast<const BatchRecord *>(d + counters_bytes),
       reinterpret_cast<const uint64_t *>(d + counters_bytes + recs_bytes), (uint32_t)items.size(), counters,
-      counters + n_rec, counters + n_rec + 1, wait_limit_slot(counters, n_rec), device_tables_on_gpu());
+      counters + n_rec, counters + n_rec + 1, wait_limit_slot(counters, n_rec), device_tables_on_gpu(),
+      failed);
   return cudaGetLastError();
 }
 } // namespace bc
@@ -666,7 +670,7 @@ extern "C" cudaError_t bc_lde_batch_noalloc(const bc_lde_job *jobs, uint32_t n_j
                                                                          counters, counters + n_rec,
                                                                          counters + n_rec + 1,
                                                                          wait_limit_slot(counters, n_rec),
-                                                                         device_tables_on_gpu());
+                                                                         device_tables_on_gpu(), nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -21,6 +21,11 @@
 // flight on it, so requests that arrive while they run wait for the next
 // launch and join it.  The batch schedule goes through a pinned staging buffer
 // and a device scratch buffer the server allocates once (two of each).
+//
+// The kernels' waits are bounded; each request on a slot and each device launch
+// has a word of pinned memory that a kernel sets when one runs out (nothing is
+// written or copied otherwise), and the completion callback then marks the
+// launch's requests failed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -57,6 +62,9 @@ struct Request {
   size_t arena_off = 0, arena_bytes = 0;
   bool device = false; // buffers in device memory (bc_lde_server_submit_device)
 };
+
+constexpr uint32_t MAX_DEV_LAUNCHES = 1024;                  // device launches in flight
+constexpr cudaError_t WAIT_RAN_OUT = cudaErrorLaunchTimeout; // error of a request one of whose kernels' waits ran out
 
 // First-fit allocator over the device arena (offsets, 256-byte granules).
 struct Arena {
@@ -133,6 +141,8 @@ struct bc_lde_server {
   int stage_next = 0;
   int dev_in_flight = 0;
   uint64_t dev_running = 0;
+  uint32_t *wait_words = nullptr;  // pinned: one per slot, then MAX_DEV_LAUNCHES for device launches
+  std::vector<uint32_t> dev_words; // those not in use by a launch
   uint64_t max_batch_elems = 1ull << 22; // 0: every device request as its own fused LDE
   uint64_t dev_batches = 0, dev_batched_requests = 0, dev_single_requests = 0;
   uint64_t next_id = 1;
@@ -153,6 +163,7 @@ namespace {
 struct DoneCtx {
   bc_lde_server *srv;
   Request *req;
+  const volatile uint32_t *failed;
 };
 
 // Runs on a CUDA driver thread when the request's stream reaches its end;
@@ -162,7 +173,8 @@ void CUDART_CB on_request_done(void *p) {
   {
     std::lock_guard<std::mutex> lock(d->srv->mu);
     d->req->finish = Clock::now();
-    d->req->state = DONE;
+    d->req->state = *d->failed ? FAILED : DONE;
+    if (*d->failed) d->req->error = WAIT_RAN_OUT;
   }
   d->srv->cv.notify_all();
   d->srv->done_cv.notify_all();
@@ -234,11 +246,13 @@ bool admit_one(bc_lde_server *s, std::unique_lock<std::mutex> &lock) {
   r->start = Clock::now();
   lock.unlock(); // enqueue without holding the lock (the done callback takes it)
   HostPipe &hp = s->pipes[slot];
+  uint32_t *failed = s->wait_words + slot;
+  *failed = 0;
   const uint64_t n = 1ull << r->log_n;
   cudaError_t e = host_lde_enqueue(hp, r->in, r->out, r->log_n, r->cols, n, n, (uint64_t)r->cols * n, r->log_blowup,
-                                   s->arena_base + off / 8, chunk, false, nullptr);
+                                   s->arena_base + off / 8, chunk, false, nullptr, failed);
   if (e == cudaSuccess) {
-    DoneCtx *d = new (std::nothrow) DoneCtx{s, r};
+    DoneCtx *d = new (std::nothrow) DoneCtx{s, r, failed};
     e = d ? cudaLaunchHostFunc(hp.s_out, on_request_done, d) : cudaErrorMemoryAllocation;
     if (e != cudaSuccess) delete d; // never handed to the stream
   }
@@ -265,6 +279,7 @@ struct GroupCtx {
   bc_lde_server *srv;
   std::vector<Request *> reqs;
   cudaEvent_t done = nullptr;
+  uint32_t word = 0; // its wait word
 };
 
 void CUDART_CB on_group_done(void *p) {
@@ -272,11 +287,16 @@ void CUDART_CB on_group_done(void *p) {
   {
     std::lock_guard<std::mutex> lock(g->srv->mu);
     const Clock::time_point now = Clock::now();
+    const bool failed = *(const volatile uint32_t *)(g->srv->wait_words + g->word) != 0;
     for (Request *r : g->reqs) {
       r->finish = now;
-      r->state = DONE;
-      book_done(g->srv, r);
+      r->state = failed ? FAILED : DONE;
+      if (failed)
+        r->error = WAIT_RAN_OUT;
+      else
+        book_done(g->srv, r);
     }
+    g->srv->dev_words.push_back(g->word);
     g->srv->dev_running -= g->reqs.size();
     g->srv->dev_in_flight--;
     g->srv->dead_events.push_back(g->done);
@@ -294,7 +314,11 @@ void launch_device_group(bc_lde_server *s, std::vector<Request *> group, bool ba
                          std::unique_lock<std::mutex> &lock) {
   const int stage = s->stage_next;
   if (batch) s->stage_next ^= 1;
+  const uint32_t word = s->dev_words.back();
+  s->dev_words.pop_back();
   lock.unlock();
+  uint32_t *failed = s->wait_words + word;
+  *failed = 0;
   cudaError_t e = cudaSuccess;
   if (batch) {
     // the staging buffer's previous copy (two launches ago) must have completed
@@ -307,13 +331,13 @@ void launch_device_group(bc_lde_server *s, std::vector<Request *> group, bool ba
     }
     if (e == cudaSuccess)
       e = batch_enqueue_into(jobs.data(), (uint32_t)jobs.size(), s->d_sched[stage], s->h_stage[stage],
-                             SERVER_SCHED_BYTES, s->s_dev);
+                             SERVER_SCHED_BYTES, s->s_dev, failed);
     if (e == cudaSuccess) e = cudaEventRecord(s->stage_done[stage], s->s_dev);
   } else {
     const Request &r = *group[0];
     const uint64_t n = 1ull << r.log_n;
     e = lde_fused(call_plan(r.log_n, r.log_blowup, r.cols), r.in, r.out, r.log_n, r.cols, n, n,
-                  (uint64_t)r.cols * n, r.log_blowup, s->s_dev);
+                  (uint64_t)r.cols * n, r.log_blowup, s->s_dev, nullptr, 0, failed);
   }
   GroupCtx *g = nullptr;
   cudaEvent_t done = nullptr;
@@ -321,7 +345,7 @@ void launch_device_group(bc_lde_server *s, std::vector<Request *> group, bool ba
   if (e == cudaSuccess) e = cudaEventRecord(done, s->s_dev);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s->s_cb, done, 0);
   if (e == cudaSuccess) {
-    g = new (std::nothrow) GroupCtx{s, group, done};
+    g = new (std::nothrow) GroupCtx{s, group, done, word};
     e = g ? cudaLaunchHostFunc(s->s_cb, on_group_done, g) : cudaErrorMemoryAllocation;
     if (e != cudaSuccess) {
       delete g;
@@ -341,6 +365,7 @@ void launch_device_group(bc_lde_server *s, std::vector<Request *> group, bool ba
       r->state = FAILED;
       r->finish = now;
     }
+    s->dev_words.push_back(word);
     s->dev_running -= group.size();
     s->dev_in_flight--;
     s->done_cv.notify_all();
@@ -359,6 +384,8 @@ void dispatch_device(bc_lde_server *s, std::unique_lock<std::mutex> &lock) {
       // a schedule holds about 8 bytes per 4096-element work item and kernel: stop well before the scratch is full
       const uint64_t items = 4 * ((((uint64_t)r->cols << r->log_n) + 4095) / 4096) << r->log_blowup;
       if (batchable && !small.empty() && (small_items + items) * 8 > SERVER_SCHED_BYTES / 2) break;
+      // a wait word for each launch: the batch's, one for each big request
+      if (s->dev_in_flight + 1 + big.size() >= MAX_DEV_LAUNCHES) break;
       s->pending_dev.pop_front();
       r->state = RUNNING;
       r->start = Clock::now();
@@ -435,6 +462,8 @@ extern "C" cudaError_t bc_lde_server_create(const bc_lde_server_config *cfg, bc_
   }
   e = cudaStreamCreateWithFlags(&s->s_dev, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->s_cb, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMallocHost(&s->wait_words, (cfg->slots + MAX_DEV_LAUNCHES) * sizeof(uint32_t));
+  for (uint32_t w = 0; w < MAX_DEV_LAUNCHES; w++) s->dev_words.push_back(cfg->slots + w);
   for (int i = 0; i < 2 && e == cudaSuccess; i++) {
     e = cudaMalloc(&s->d_sched[i], SERVER_SCHED_BYTES);
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_stage[i], SERVER_SCHED_BYTES);
@@ -446,6 +475,7 @@ extern "C" cudaError_t bc_lde_server_create(const bc_lde_server_config *cfg, bc_
       cudaFreeHost(s->h_stage[i]);
       cudaFree(s->d_sched[i]);
     }
+    cudaFreeHost(s->wait_words);
     if (s->s_dev) cudaStreamDestroy(s->s_dev);
     if (s->s_cb) cudaStreamDestroy(s->s_cb);
     for (auto &q : s->pipes) host_pipe_destroy(q);
@@ -647,6 +677,7 @@ extern "C" cudaError_t bc_lde_server_destroy(bc_lde_server *s) {
     cudaFreeHost(s->h_stage[i]);
     cudaFree(s->d_sched[i]);
   }
+  cudaFreeHost(s->wait_words);
   cudaStreamDestroy(s->s_dev);
   cudaStreamDestroy(s->s_cb);
   cudaFree(s->arena_base);

@@ -307,7 +307,9 @@ cudaError_t bc_lde_server_set_device_batching(bc_lde_server *server, uint64_t ma
  * device requests run as their own fused LDE. */
 cudaError_t bc_lde_server_get_device_stats(bc_lde_server *server, uint64_t *batches, uint64_t *batched_requests,
                                            uint64_t *single_requests);
-/* *state: 0 pending, 1 running, 2 done, 3 cancelled, 4 failed (the call returns the error). */
+/* *state: 0 pending, 1 running, 2 done, 3 cancelled, 4 failed (the call returns the error:
+ * that of enqueuing it, or cudaErrorLaunchTimeout when a bounded wait of its kernels ran out
+ * and its outputs are invalid; served requests report that here, not in bc_ntt_wait_status). */
 cudaError_t bc_lde_server_poll(bc_lde_server *server, uint64_t request_id, int *state, double *latency_ms);
 /* Waits up to timeout_ms: cudaErrorTimeout if still unfinished, cudaErrorNotReady if cancelled. */
 cudaError_t bc_lde_server_wait(bc_lde_server *server, uint64_t request_id, uint32_t timeout_ms, double *latency_ms);

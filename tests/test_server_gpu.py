@@ -153,3 +153,64 @@ def test_server_device_requests_equal_alone(gpu_ctx, max_batch_elems):
         assert st["batches"] >= 1 and st["batched_requests"] >= 2
     else:
         assert st["batches"] == 0
+
+
+@pytest.mark.parametrize("mode", ["batched", "single", "host"])
+def test_server_fails_requests_whose_waits_run_out(gpu_ctx, mode):
+    """With a limit of no tries the kernels' waits for products run out: every request of such a launch ends as
+    failed, not as done, and nothing else does; with the default again, the same requests are done and exact."""
+    import bc_ntt
+    import torch
+
+    rng = np.random.default_rng(606)
+    srv = bc_ntt.LdeServer(memory_budget_bytes=256 << 20, slots=2)
+    srv.set_device_batching(1 << 22 if mode == "batched" else 0)
+    specs = [(14, 17, 1), (16, 4, 2), (13, 16, 1), (17, 8, 1)]
+    xs = [raw_u64(rng, cols << log_n) for log_n, cols, _ in specs]
+    if mode == "host":
+        ins = [_pinned(x) for x in xs]
+        outs = [_pinned(np.zeros(x.size << b, dtype=np.uint64)) for x, (_, _, b) in zip(xs, specs)]
+    else:
+        ins = [to_dev(x) for x in xs]
+        outs = [torch.zeros(x.size << b, dtype=torch.int64, device="cuda") for x, (_, _, b) in zip(xs, specs)]
+    submit = srv.submit if mode == "host" else srv.submit_device
+
+    def submit_all():
+        return [submit(i, o, *spec) for i, o, spec in zip(ins, outs, specs)]
+
+    try:
+        bc_ntt.set_wait_limit(0)
+        for rid in submit_all():
+            with pytest.raises(RuntimeError, match="702"):  # cudaErrorLaunchTimeout
+                srv.wait(rid, timeout_ms=60000)
+            with pytest.raises(RuntimeError, match="702"):
+                srv.poll(rid)
+            assert srv.release(rid) is True
+        assert srv.stats()["completed"] == 0
+    finally:
+        bc_ntt.set_wait_limit()
+    assert bc_ntt.wait_status() == 0  # reported by the requests
+    for rid in submit_all():
+        srv.wait(rid, timeout_ms=60000)
+    assert srv.stats()["completed"] == len(specs)
+    srv.close()
+    for x, o, (log_n, cols, log_b) in zip(xs, outs, specs):
+        got = o.numpy().view(np.uint64) if mode == "host" else to_host(o)
+        np.testing.assert_array_equal(got, _alone(x, log_n, cols, log_b))
+
+
+def test_server_more_big_requests_than_launches_in_flight(gpu_ctx):
+    """Big device requests beyond the launches that may be in flight wait their turn."""
+    import bc_ntt
+    import torch
+
+    srv = bc_ntt.LdeServer(memory_budget_bytes=64 << 20, slots=1)
+    srv.set_device_batching(0)
+    x = raw_u64(np.random.default_rng(1), 2 << 10)
+    d, outs = to_dev(x), torch.zeros(3000, 4 << 10, dtype=torch.int64, device="cuda")
+    ids = [srv.submit_device(d, outs[i], 10, 2, 1) for i in range(3000)]
+    for rid in ids:
+        srv.wait(rid, timeout_ms=60000)
+    assert srv.device_stats()["single_requests"] == 3000
+    srv.close()
+    assert bool((outs == to_dev(_alone(x, 10, 2, 1))).all())
