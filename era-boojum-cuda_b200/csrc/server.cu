@@ -381,9 +381,12 @@ void dispatch_device(bc_lde_server *s, std::unique_lock<std::mutex> &lock) {
     while (!s->pending_dev.empty()) {
       Request *r = s->pending_dev.front();
       const bool batchable = s->max_batch_elems && out_elems(*r) <= s->max_batch_elems;
-      // a schedule holds about 8 bytes per 4096-element work item and kernel: stop well before the scratch is full
+      // a schedule holds about 8 bytes per 4096-element work item and kernel, and fewer than 2^16 kernels (seven a
+      // request at most): stop well before the scratch is full or the numbers run out
       const uint64_t items = 4 * ((((uint64_t)r->cols << r->log_n) + 4095) / 4096) << r->log_blowup;
-      if (batchable && !small.empty() && (small_items + items) * 8 > SERVER_SCHED_BYTES / 2) break;
+      if (batchable && !small.empty() &&
+          ((small_items + items) * 8 > SERVER_SCHED_BYTES / 2 || small.size() >= 8192))
+        break;
       // a wait word for each launch: the batch's, one for each big request
       if (s->dev_in_flight + 1 + big.size() >= MAX_DEV_LAUNCHES) break;
       s->pending_dev.pop_front();

@@ -214,3 +214,25 @@ def test_server_more_big_requests_than_launches_in_flight(gpu_ctx):
     assert srv.device_stats()["single_requests"] == 3000
     srv.close()
     assert bool((outs == to_dev(_alone(x, 10, 2, 1))).all())
+
+
+def test_server_many_tiny_requests_pending(gpu_ctx):
+    """More pending small requests than one batch's schedule can number: they take several launches."""
+    import bc_ntt
+    import torch
+
+    srv = bc_ntt.LdeServer(memory_budget_bytes=64 << 20, slots=1)
+    big = torch.zeros(64 << 22, dtype=torch.int64, device="cuda")
+    big_out = torch.zeros(128 << 22, dtype=torch.int64, device="cuda")
+    x = raw_u64(np.random.default_rng(2), 1 << 13)
+    d, outs = to_dev(x), torch.zeros(30000, 2 << 13, dtype=torch.int64, device="cuda")
+    heads = [srv.submit_device(big, big_out, 22, 64, 1) for _ in range(40)]  # keeps the device busy meanwhile
+    ids = []
+    for i in range(30000):
+        ids.append(srv.submit_device(d, outs[i], 13, 1, 1))
+    for rid in heads + ids:
+        srv.wait(rid, timeout_ms=60000)
+    st = srv.device_stats()
+    assert st["batched_requests"] + st["single_requests"] == len(heads) + len(ids)
+    srv.close()
+    assert bool((outs == to_dev(_alone(x, 13, 1, 1))).all())
