@@ -192,6 +192,7 @@ def test_server_fails_requests_whose_waits_run_out(gpu_ctx, mode):
     assert bc_ntt.wait_status() == 0  # reported by the requests
     for rid in submit_all():
         srv.wait(rid, timeout_ms=60000)
+        assert srv.release(rid) is True  # a host request is booked when it is retired, here at the latest
     assert srv.stats()["completed"] == len(specs)
     srv.close()
     for x, o, (log_n, cols, log_b) in zip(xs, outs, specs):
