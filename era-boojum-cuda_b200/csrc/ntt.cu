@@ -239,30 +239,37 @@ cudaError_t context_destroy_current() {
 }
 
 // ---------------------------------------------------------------- plans
+static Plan two_pass(int top, int low) {
+  Plan pl{};
+  pl.npasses = 2;
+  pl.pass[0] = {(uint8_t)top, (uint8_t)(top <= 9 ? 8 : top == 10 ? 4 : 2)};
+  pl.pass[1] = {(uint8_t)low, 1};
+  return pl;
+}
+
 // Default pass plans.  The pass that owns bit 0 takes up to 12 bits (contiguous
 // 32 KB tiles); the others use windows whose shared-memory rounds are free of
 // bank conflicts: 4, 5, 8 or 9 bits with runs of 8 (64-byte rows), 10 bits with
-// runs of 4, 11 bits with runs of 2.
+// runs of 4, 11 bits with runs of 2.  On the tensor cores a window of 4 j + 1
+// bits spends a round on its last bit: upper windows of 5 and 9 bits lost to 4
+// and 8 (B200, plain forward: 64 x 2^14 21.0 us as 5 + 9, 19.0 as 4 + 10; 16 x
+// 2^18 86 as 9 + 9, 76 as 8 + 10), and on the other kernels these splits are no
+// slower at 18..20 bits.
 Plan default_plan(uint32_t log_n) {
   Plan pl{};
-  auto run_for = [](int K) -> uint8_t { return K <= 9 ? 8 : K == 10 ? 4 : 2; };
-  // top window bits for 13..23 (index log_n - 13), then 12 bits at the bottom
-  static const uint8_t top2[11] = {5, 5, 5, 8, 8, 9, 9, 9, 9, 10, 11};
-  static const uint8_t low2[11] = {8, 9, 10, 8, 9, 9, 10, 11, 12, 12, 12};
+  // top window bits for 13..23 (index log_n - 13)
+  static const uint8_t top2[11] = {5, 4, 4, 8, 8, 8, 8, 8, 9, 10, 11};
   if (log_n <= 12) {
     pl.npasses = 1;
     pl.pass[0] = {(uint8_t)log_n, 1};
   } else if (log_n <= 23) {
-    pl.npasses = 2;
-    const int k1 = top2[log_n - 13], k2 = low2[log_n - 13];
-    pl.pass[0] = {(uint8_t)k1, run_for(k1)};
-    pl.pass[1] = {(uint8_t)k2, 1};
+    pl = two_pass(top2[log_n - 13], (int)log_n - top2[log_n - 13]);
   } else {
     // 24..27: two upper windows from {4, 5, 8, 9, 10} over the bits above 12
     static const uint8_t a3[4] = {4, 5, 5, 5}, b3[4] = {8, 8, 9, 10};
     pl.npasses = 3;
-    pl.pass[0] = {a3[log_n - 24], run_for(a3[log_n - 24])};
-    pl.pass[1] = {b3[log_n - 24], run_for(b3[log_n - 24])};
+    pl.pass[0] = {a3[log_n - 24], 8};
+    pl.pass[1] = {b3[log_n - 24], (uint8_t)(b3[log_n - 24] == 10 ? 4 : 8)};
     pl.pass[2] = {12, 1};
   }
   return pl;
@@ -271,29 +278,85 @@ Plan default_plan(uint32_t log_n) {
 // A plan whose lowest window is below 12 bits tiles columns together on the
 // tensor cores (2^(12 - K) of them).  With fewer columns than fill such a tile
 // (tc_window_ok) that pass, and with it the fused top window, would run on the
-// other kernels: a two-pass split with the next larger low window that is
-// filled is taken instead, 12 bits at most (B200, 2 x 2^22 plain: 3 passes on
-// the other kernels against 2 here), else one bit more in the low window
-// (2^13: 4 + 9 bits instead of 5 + 8, 6 % faster on the other kernels).
-Plan fit_plan(const Plan &pl, uint32_t log_n, uint32_t cols) {
+// other kernels: a two-pass split with a larger low window that is filled is
+// taken instead, 12 bits at most, else one bit more in the low window (2^13: 4
+// + 9 bits instead of 5 + 8, 6 % faster on the other kernels).  Upper windows
+// of 4, 8 or 10 bits before 5 or 9 when whole_rounds (plain transforms, 16 bits
+// as 4 + 12 against 5 + 11, 2..100 columns: 10 to 15 % faster).
+static bool fit_split(int low, uint32_t log_n, uint32_t cols, bool whole_rounds, Plan &pl) {
+  for (int any = whole_rounds ? 0 : 1; any < 2; any++)
+    for (int k = low + 1; k <= 12; k++) {
+      const int top = (int)log_n - k;
+      if ((top == 4 || top == 8 || top == 10 || (any && (top == 5 || top == 9))) && tc_window_ok(k, 0, cols, true, true)) {
+        const Knobs knobs = pl.knobs;
+        pl = two_pass(top, k);
+        pl.knobs = knobs;
+        return true;
+      }
+    }
+  return false;
+}
+static bool fit_one_more(Plan &pl) {
+  const int top = pl.pass[0].K, low = pl.pass[1].K;
+  if (pl.npasses != 2 || (top != 5 && top != 9) || low >= 12) return false;
+  const Knobs knobs = pl.knobs;
+  pl = two_pass(top - 1, low + 1);
+  pl.knobs = knobs;
+  return true;
+}
+
+Plan fit_plan(Plan pl, uint32_t log_n, uint32_t cols) {
   const int low = pl.pass[pl.npasses - 1].K;
   if (cols > 65535) return pl; // the tensor-core kernels' limit, not few
   if (pl.npasses < 2 || pl.pass[pl.npasses - 1].C != 1 || low < 8 || tc_window_ok(low, 0, cols, true, true)) return pl;
-  auto split = [&](int k) {
-    const int top = (int)log_n - k;
-    Plan q{};
-    q.npasses = 2;
-    q.pass[0] = {(uint8_t)top, (uint8_t)(top <= 9 ? 8 : 4)};
-    q.pass[1] = {(uint8_t)k, 1};
-    q.knobs = pl.knobs;
+  if (!fit_split(low, log_n, cols, false, pl)) fit_one_more(pl);
+  return pl;
+}
+
+// The same for a plain transform, where the kinds of call differ in what they
+// can run on the tensor cores.  Times on B200, of calls captured into a graph,
+// 1..100 columns of 2^13..2^21 in every mode.
+Plan fit_ntt_plan(Plan pl, uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset) {
+  if (log_n <= 12 || cols > 65535) return pl;
+  const int low = pl.pass[pl.npasses - 1].K;
+  if (low < 8 || low > 12) return pl;
+  const uint32_t g = 1u << tc_log_g(low, true), slots = (cols + g - 1) / g * g, tiles = cols << (log_n - 12);
+  // Three passes gain from a short low window only when its tiles are full: two
+  // otherwise (12 x 2^21: 428 us as 9 + 12, 476 as 4 + 8 + 9).
+  const bool two = pl.npasses < 3 || (log_n <= 22 && 8 * cols < 7 * slots);
+  // One pass of these keeps the integer kernel (tc_pass_ok): the last of a
+  // natural -> bit-reversed inverse, the first of a bit-reversed -> natural
+  // forward transform of a coset.  Columns that do not fill a tile are nothing
+  // to it, and the splits are those that suit it best (3 x 2^16 inverse: 16 us
+  // as 8 + 8, 20 as 5 + 11; of a coset, 12 x 2^13: 20 as 5 + 8, 25 as 4 + 9; 3 x
+  // 2^21: 159 as 9 + 12, 186 as 4 + 8 + 9), with three CTAs an SM in low windows
+  // of 9..11 bits (33 x 2^17: 120 against 131).
+  if (b2n != inverse && (inverse || coset)) {
+    if (!two || log_n > 22) return pl;
+    int top = (int)(log_n < 21 ? 8 : log_n - 12);
+    if (log_n < 16) top = b2n ? (log_n == 13 ? 5 : 4) : coset ? 5 : 4;
+    Plan q = two_pass(top, (int)log_n - top);
+    if (inverse && q.pass[1].K >= 9 && q.pass[1].K <= 11) q.knobs.occ = BC_PASS_MIN_BLOCKS_B2N;
     return q;
-  };
-  for (int k = low + 1; k <= 12; k++) {
-    const int top = (int)log_n - k;
-    if ((top == 4 || top == 5 || (top >= 8 && top <= 10)) && tc_window_ok(k, 0, cols, true, true)) return split(k);
   }
-  const int top = pl.pass[0].K;
-  return pl.npasses == 2 && (top == 5 || top == 9) && low < 12 ? split(low + 1) : pl;
+  if (two && pl.npasses == 3) return default_plan(log_n);
+  if (tc_window_ok(low, 0, cols, b2n, inverse)) return pl;
+  Plan q = pl;
+  if (fit_split(low, log_n, cols, true, q)) {
+    // half a wave of 12-bit tiles (5 x 2^16 forward: 15.3 us as 8 + 8, 16.5 as 4 + 12; 3 x 2^16: 15.0 and 12.2)
+    const bool half_wave = q.pass[1].K == 12 && tiles > 64 && tiles <= 128;
+    return half_wave && !b2n && !coset ? pl : q;
+  }
+  // All on the integer kernels if the coset's powers cannot be spread over the
+  // passes; their split also when the columns are more than half of the tiles
+  // under a 4-bit window (forward, 5 x 2^13: 11.8 us as 5 + 8, 12.8 as 4 + 9; of
+  // a coset 13 and 15).
+  if (!b2n && log_n <= 15) {
+    const uint32_t g4 = 1u << tc_log_g((int)log_n - 4, true), slots4 = (cols + g4 - 1) / g4 * g4;
+    if (coset || 2 * cols > slots4) return two_pass(5, (int)log_n - 5);
+  }
+  fit_one_more(pl);
+  return pl;
 }
 
 static bool shape_supported(int K, int C) {
@@ -493,6 +556,36 @@ cudaError_t launch_pass(const PassLaunch &pl, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// Whether pass i of a plain transform gains from the tensor-core kernel.
+static bool tc_faster(const Plan &pl, int i, uint32_t cols, bool b2n, bool inverse, bool scaled) {
+  const int K = pl.pass[i].K;
+  if (pl.npasses == 1) {
+    // A single pass has index prefix 0: the integer kernels skip the top
+    // round's powers, and nothing hides this kernel's tables.  Measured at 1 to
+    // 30000 columns of 2^8..2^12 (ratio of times, tensor cores / integer):
+    // inverse 0.63-1.0; forward with a coset 1.0-1.15 up to a CTA an SM, then
+    // 0.77-1.0; plain forward, natural -> bit-reversed, 1.0-1.36 (12 bits: 0.96
+    // from some 4000 columns on), bit-reversed -> natural 1.0-1.2 with 9 bits,
+    // 0.76-0.96 with 12, else 1.0-1.12 up to about 1000 tiles, then 0.87-1.0.
+    const uint32_t g = 1u << tc_log_g(K, true), tiles = (cols + g - 1) / g;
+    if (inverse) return true;
+    if (scaled) return tiles > (uint32_t)sm_count();
+    if (!b2n) return K == 12 && tiles > 2048;
+    return K == 12 || (K != 9 && tiles > 1024);
+  }
+  // Upper windows of a plain natural -> bit-reversed transform that end in a
+  // round of one bit: with 9 bits the integer kernel is up to 10 % faster (8 x
+  // 2^18, 3 x 2^21), with 5 bits up to 16 % (64 x 2^15) unless the next pass is a
+  // tensor-core one, whose tables are then built meanwhile (33 x 2^14: 12 % for
+  // the tensor cores).  Scaled by a coset's powers they gain, as windows that
+  // are whole rounds do.
+  if (!b2n && !scaled && i + 1 < pl.npasses) {
+    if (K == 9) return false;
+    if (K == 5 && i + 2 == pl.npasses) return tc_window_ok(pl.pass[i + 1].K, 0, cols, b2n, inverse);
+  }
+  return true;
+}
+
 cudaError_t launch_ntt(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_ntts,
                        uint64_t stride_in, uint64_t stride_out, bool bitrev_inputs, bool inverse, uint32_t log_ext,
                        uint32_t coset_idx, cudaStream_t stream) {
@@ -502,9 +595,12 @@ cudaError_t launch_ntt(const Plan &pl, const uint64_t *in, uint64_t *out, uint32
   // the tensor cores, and otherwise applied whole by its first (forward) or
   // last (inverse) pass
   const bool scaled = log_ext > 0 && bitrev_inputs == inverse;
-  bool share = scaled;
-  for (int i = 0; share && i < pl.npasses; i++)
-    share = tc_window_ok(pl.pass[i].K, plan_lb(pl, log_n, i), num_ntts, bitrev_inputs, inverse);
+  bool on_tc[4], share = scaled;
+  for (int i = 0; i < pl.npasses; i++) {
+    on_tc[i] = tc_window_ok(pl.pass[i].K, plan_lb(pl, log_n, i), num_ntts, bitrev_inputs, inverse) &&
+               tc_faster(pl, i, num_ntts, bitrev_inputs, inverse, scaled);
+    share = share && on_tc[i];
+  }
   bool prev_tc = false;
   for (int s = 0; s < pl.npasses; s++) {
     const int i = bitrev_inputs ? pl.npasses - 1 - s : s; // b2n runs the passes bottom-up
@@ -530,7 +626,7 @@ cudaError_t launch_ntt(const Plan &pl, const uint64_t *in, uint64_t *out, uint32
     q.walk = plan_walk(pl);
     q.occ = pl.knobs.occ;
     q.overlap = prev_tc;
-    prev_tc = q.tc = tc_pass_ok(q);
+    prev_tc = q.tc = on_tc[i] && tc_pass_ok(q);
     cudaError_t e = launch_pass(q, stream);
     if (e != cudaSuccess) return e;
   }
@@ -577,8 +673,9 @@ extern "C" cudaError_t bc_batch_ntt_internal(const uint64_t *inputs, uint64_t *o
                                              uint32_t coset_index, cudaStream_t stream) {
   if (!ntt_args_ok(log_n, stride_in, stride_out, log_extension_degree, coset_index)) return cudaErrorInvalidValue;
   if (num_ntts && (!inputs || !outputs)) return cudaErrorInvalidValue;
-  return launch_ntt(call_plan(log_n, 0, num_ntts), inputs, outputs, log_n, num_ntts, stride_in, stride_out,
-                    bitrev_inputs, inverse, log_extension_degree, coset_index, stream);
+  const Plan pl = call_ntt_plan(log_n, num_ntts, bitrev_inputs, inverse, log_extension_degree > 0);
+  return launch_ntt(pl, inputs, outputs, log_n, num_ntts, stride_in, stride_out, bitrev_inputs, inverse,
+                    log_extension_degree, coset_index, stream);
 }
 
 extern "C" cudaError_t bc_batch_ntt_out_of_place(const uint64_t *inputs_matrix, size_t inputs_len,

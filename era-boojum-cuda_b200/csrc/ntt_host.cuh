@@ -68,13 +68,14 @@ int current_device();
 int sm_count();
 
 Plan default_plan(uint32_t log_n);
-// The plan, or one with a larger low window for few columns.
-Plan fit_plan(const Plan &pl, uint32_t log_n, uint32_t cols);
-// The plan of a call for an LDE (log_blowup >= 1) or a plain NTT (log_blowup =
-// 0) on the current device (tune.cu): an entry that the caller imported or
-// autotuned, as it is; else the default entry of the table or, without one,
-// default_plan, either fitted to the columns.
+// The plan, or one that suits the columns (and kind of transform) better.
+Plan fit_plan(Plan pl, uint32_t log_n, uint32_t cols);
+Plan fit_ntt_plan(Plan pl, uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset);
+// The plan of an LDE and of a plain NTT on the current device (tune.cu): an
+// entry that the caller imported or autotuned, as it is; else the default entry
+// of the table or, without one, default_plan, either fitted to the call.
 Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols);
+Plan call_ntt_plan(uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset);
 bool plan_valid(const Plan &pl, uint32_t log_n);
 
 // Scaling by base^i, i the natural index, spread over the passes: the index is

@@ -23,9 +23,16 @@ cudaError_t tc_fill_images(uint8_t *img) {
   return cudaGetLastError();
 }
 
+// A natural -> bit-reversed inverse scales by bit-reversed indexes in its pass at
+// bit 0, which is not this kernel's, and does not gain from it with 9 bits above
+// (launch_ntt): no instances.
 template <int K, bool LOW> static PassKernel tk(bool b2n, bool inverse) {
   if (b2n) return inverse ? tc::pass_kernel_tc<K, LOW, true, true> : tc::pass_kernel_tc<K, LOW, true, false>;
-  return inverse ? tc::pass_kernel_tc<K, LOW, false, true> : tc::pass_kernel_tc<K, LOW, false, false>;
+  if (!inverse) return tc::pass_kernel_tc<K, LOW, false, false>;
+  if constexpr (!LOW && K != 9)
+    return tc::pass_kernel_tc<K, LOW, false, true>;
+  else
+    return nullptr;
 }
 
 PassKernel pick_pass_kernel_tc(int K, bool low, bool b2n, bool inverse) {

@@ -17,7 +17,7 @@
 // Entries are of two kinds.  What the caller imported or autotuned is run as it
 // is, whatever the columns.  Default entries (bc_plan_table_import_defaults:
 // the shipped table) stand in for built-in plans and, like these, are fitted
-// to calls of few columns (fit_plan).
+// to the call (fit_plan, fit_ntt_plan).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -122,15 +122,24 @@ const KnobAxis KNOB_AXES[] = {
 };
 } // namespace
 
-Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols) {
-  Entry en{default_plan(log_n), true};
+static Entry entry_of(uint32_t log_n, uint32_t log_blowup) {
   const int d = current_device();
   if (d >= 0 && d < TUNE_MAX_DEVICES) {
     std::lock_guard<std::mutex> lock(g_table_mutex);
     auto it = g_table[d].find(key(log_n, log_blowup));
-    if (it != g_table[d].end()) en = it->second;
+    if (it != g_table[d].end()) return it->second;
   }
+  return Entry{default_plan(log_n), true};
+}
+
+Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols) {
+  const Entry en = entry_of(log_n, log_blowup);
   return en.fit ? fit_plan(en.plan, log_n, cols) : en.plan;
+}
+
+Plan call_ntt_plan(uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset) {
+  const Entry en = entry_of(log_n, 0);
+  return en.fit ? fit_ntt_plan(en.plan, log_n, cols, b2n, inverse, coset) : en.plan;
 }
 
 } // namespace bc

@@ -103,9 +103,9 @@ cudaError_t bc_batch_ntt_with_plan(const uint64_t *inputs, uint64_t *outputs, ui
  * Each device keeps a table keyed by (log_n, log_blowup), log_blowup = 0 for
  * the plain NTT; every entry point here uses the table's plan when present and
  * the built-in one otherwise.  A plan that the caller imported or autotuned runs
- * as it is, whatever the columns; built-in plans, and those imported as
- * defaults, may be replaced by one with a larger low window for calls with too
- * few columns to fill theirs.  bc_autotune times every candidate plan on the
+ * as it is, whatever the call; built-in plans, and those imported as defaults,
+ * may be replaced by one that suits a call's columns or kind of transform
+ * better.  bc_autotune times every candidate plan on the
  * current device (num_cols columns, reps timed runs after one warm-up; it
  * allocates and frees its own scratch and synchronises), then the launch knobs
  * of the fastest window split one at a time (column-group walk of the pass and

@@ -4,7 +4,7 @@ index, short rounds, column counts around a tile's, cosets, odd strides."""
 import numpy as np
 import pytest
 
-from conftest import raw_u64, to_dev, to_host
+from conftest import kernel_names, raw_u64, to_dev, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -185,3 +185,92 @@ def test_waits_that_run_out_are_reported(gpu_ctx, log_n, cols, log_b, plan):
         bc_ntt.plan_table_clear()
         if old:
             bc_ntt.plan_table_import(old)
+
+
+MODES = [(False, False), (False, True), (True, False), (True, True)]
+
+
+@pytest.mark.parametrize("low", [8, 9, 10, 11, 12])
+@pytest.mark.parametrize("bitrev,inverse", MODES)
+def test_low_windows_below_a_top_window(gpu_ctx, low, bitrev, inverse):
+    """The low windows with index prefixes, on the tensor cores but for the last pass of a natural -> bit-reversed
+    inverse and the first of a scaled bit-reversed -> natural forward transform."""
+    import bc_ntt
+
+    plan, log_n, g = [(4, 8), (low, 1)], 4 + low, 1 << (12 - low)
+    for cols in {1, max(1, 3 * g // 4), g, g + max(1, 3 * g // 4)}:
+        _ntt(log_n, cols, bitrev, inverse, plan=plan)
+        for ext in (0, 1):
+            n = 1 << log_n
+            d = to_dev(np.zeros(cols * n, dtype=np.uint64))
+            names = kernel_names(lambda: bc_ntt.batch_ntt_with_plan(d, d, log_n, cols, n, n, bitrev, inverse, ext, ext, plan))
+            filled = 4 * cols >= 3 * g * -(-cols // g)
+            mixed = bitrev != inverse and (inverse or ext)
+            assert any(k.startswith(f"pass_kernel_tc<{low},1") for k in names) == (filled and not mixed), (cols, ext)
+    _ntt(log_n, g, bitrev, inverse, gap=3, plan=plan)
+    if bitrev == inverse:
+        _ntt(log_n, g, bitrev, inverse, ext=2, coset=3, gap=1, plan=plan)
+
+
+def _windows(log_n, cols, bitrev, inverse, ext):
+    """Windows of a plain transform's kernels, the largest first: t8 on the tensor cores, i8 on the integer kernels."""
+    import torch
+
+    import bc_ntt
+
+    n = 1 << log_n
+    d = torch.zeros(cols * n, dtype=torch.int64, device="cuda")
+    names = kernel_names(lambda: bc_ntt.batch_ntt_internal(d.data_ptr(), d.data_ptr(), log_n, cols, n, n, bitrev, inverse,
+                                                           ext, ext))
+    return sorted((("t" if k.startswith("pass_kernel_tc") else "i") + k.split("<")[1].split(",")[0] for k in names),
+                  key=lambda w: -int(w[1:]))
+
+
+# calls on both sides of each rule that chooses a plan or a kernel: (log_n, columns, bitrev, inverse, coset), windows
+ROUTES = [
+    # one pass: forward on the integer kernels up to a size, inverse on the tensor cores where the tile is filled
+    ((12, 16, 0, 0, 0), "i12"), ((12, 3000, 0, 0, 0), "t12"), ((11, 8000, 0, 0, 0), "i11"), ((12, 16, 1, 0, 0), "t12"),
+    ((9, 8000, 1, 0, 0), "i9"), ((10, 400, 1, 0, 0), "i10"), ((10, 5000, 1, 0, 0), "t10"), ((12, 100, 0, 0, 1), "i12"),
+    ((12, 200, 0, 0, 1), "t12"), ((12, 1, 1, 1, 0), "t12"), ((10, 2, 1, 1, 1), "i10"), ((10, 3, 1, 1, 1), "t10"),
+    # low windows that the columns do or do not fill
+    ((13, 16, 0, 0, 0), "t8 t5"), ((13, 5, 0, 0, 0), "i8 i5"), ((13, 3, 0, 0, 0), "i9 t4"), ((13, 1, 0, 0, 1), "i8 i5"),
+    ((13, 1, 1, 1, 1), "i9 i4"), ((13, 3, 1, 1, 0), "i9 t4"), ((14, 4, 0, 0, 1), "t10 t4"), ((14, 5, 0, 0, 1), "i9 i5"),
+    ((16, 3, 0, 0, 0), "t12 t4"), ((16, 5, 0, 0, 0), "t8 i8"), ((16, 5, 0, 0, 1), "t12 t4"), ((16, 16, 0, 0, 0), "t8 t8"),
+    ((17, 5, 0, 0, 0), "t12 t5"), ((18, 16, 0, 0, 0), "t10 t8"), ((21, 3, 0, 0, 0), "t12 i9"), ((21, 3, 0, 0, 1), "t12 t9"),
+    # a pass that keeps the integer kernel
+    ((13, 12, 0, 1, 1), "i8 i5"), ((13, 12, 0, 1, 0), "i9 t4"), ((13, 12, 1, 0, 1), "i8 t5"), ((15, 3, 0, 1, 1), "i10 i5"),
+    ((16, 3, 0, 1, 0), "t8 i8"), ((16, 3, 1, 0, 1), "t8 i8"), ((18, 33, 0, 1, 1), "i10 t8"), ((21, 3, 0, 1, 0), "i12 i9"),
+    ((22, 3, 0, 1, 1), "i12 t10"),
+]
+
+
+@pytest.mark.parametrize("call,windows", ROUTES, ids=lambda x: "-".join(map(str, x)) if isinstance(x, tuple) else None)
+def test_routes(gpu_ctx, call, windows):
+    """The kernels that a call with built-in plans takes, and its result against the oracle's."""
+    import bc_ntt
+
+    log_n, cols, bitrev, inverse, ext = call
+    old = bc_ntt.plan_table_export()
+    try:
+        bc_ntt.plan_table_clear()
+        got = _windows(log_n, cols, bool(bitrev), bool(inverse), ext)
+        assert sorted(got) == sorted(windows.split()), got
+        if cols << log_n <= 1 << 21:
+            _ntt(log_n, cols, bool(bitrev), bool(inverse), ext=ext, coset=ext)
+    finally:
+        if old:
+            bc_ntt.plan_table_import(old)
+
+
+def test_three_pass_routes(gpu_ctx):
+    """The shipped table's three-pass plans at 21 bits: for full tiles, otherwise two passes."""
+    import bc_ntt
+
+    try:
+        assert bc_ntt.load_tuned_plans()
+        assert sorted(_windows(21, 16, False, False, 0)) == ["t4", "t8", "t9"]
+        assert sorted(_windows(21, 12, False, False, 0)) == ["i9", "t12"]
+        assert sorted(_windows(21, 16, False, True, 1)) == ["i9", "t4", "t8"]
+        assert sorted(_windows(21, 12, False, True, 1)) == ["i12", "i9"]
+    finally:
+        bc_ntt.plan_table_clear()
