@@ -381,7 +381,9 @@ __device__ __forceinline__ void pass_body_tc(const PassParams &p, uint32_t bx, u
     if (more) first(c0 + G); // the operands have been read: the tile is free
     // straight from registers: neighbouring threads write neighbouring addresses,
     // or (DIT, bit 0, short last round) a thread its row's runs of 2^V words, 16
-    // bytes at a time (10-bit passes: 10 % faster than through the tile)
+    // bytes at a time (10-bit passes: 10 % faster than through the tile), the
+    // threads' runs one after the other
+    static_assert(rows_ascend(RS::make(B2N, LAST)), "neighbouring threads store to neighbouring addresses");
     uint64_t *dst = elem_at<K, LC>(out + (uint64_t)c0 * p.stride_out, e_out, p.stride_out, step_bytes);
     uint64_t even = 0;
     outputs(ctx, [&](int o, uint64_t y) {

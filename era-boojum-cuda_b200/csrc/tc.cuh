@@ -235,6 +235,14 @@ __host__ __device__ constexpr bool spans16(int a, int b, int c, int d) {
   return seen == 0xffff;
 }
 
+// Whether the rows of a layout count its other tile index bits upwards, so that
+// neighbouring threads hold neighbouring elements.
+__host__ __device__ constexpr bool rows_ascend(const Layout &q) {
+  for (int i = 0; i < 7; i++)
+    if (q.row[i] >= q.row[i + 1]) return false;
+  return true;
+}
+
 template <int K, int LC> struct Rounds {
   static constexpr int R = K % 4, NF = K / 4, N = NF + (R ? 1 : 0);
   // layout of round i of the execution order, row order as the bank rule of the
@@ -253,15 +261,6 @@ template <int K, int LC> struct Rounds {
     for (int b = 0; b < TILE_BITS; b++)
       if (!in4(q.slot, b)) rest[nrow++] = b;
     for (int t = 0; t < 8; t++) q.row[t] = rest[t];
-    if (i + 1 == N && is_short && LC == 0) {
-      // the tile is read back 16 bytes a thread: tile index bits 1..3 on three different chunk bits
-      int o = 0, n = 0;
-      for (; o < q.V - 1; n++)
-        if (rest[n] > 3) q.row[o++] = rest[n];
-      for (int t = q.V; t < 4; t++) q.row[o++] = t;
-      for (; n < 8; n++)
-        if (rest[n] > 3) q.row[o++] = rest[n];
-    }
     if (i + 1 < N) {
       const Layout n = make(dif, i + 1);
       bool found = false;
