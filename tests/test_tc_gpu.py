@@ -58,7 +58,7 @@ def test_window_plans(gpu_ctx, plan, bitrev, inverse):
 @pytest.mark.parametrize("plan", [[(4, 8), (8, 1)], [(5, 8), (8, 1)], [(8, 8), (8, 1)], [(10, 4), (8, 1)],
                                   [(4, 8), (4, 8), (8, 1)], [(5, 8), (4, 8), (9, 1)]],
                          ids=lambda p: "+".join(f"{k}.{c}" for k, c in p))
-@pytest.mark.parametrize("log_b", [1, 3, 5])
+@pytest.mark.parametrize("log_b", [1, 3, 4, 5])
 def test_lde_top_windows(gpu_ctx, plan, log_b):
     import torch
 
@@ -77,6 +77,11 @@ def test_lde_top_windows(gpu_ctx, plan, log_b):
             d, o = to_dev(x), torch.zeros(cols * n << log_b, dtype=torch.int64, device="cuda")
             bc_ntt.lde(d, o, log_n, cols, log_b)
             assert np.array_equal(to_host(o), oracle.lde(x, log_n, cols, n, log_b)), cols
+            # the top window runs on the tensor cores up to blowup 16, where the low one's tiles are filled
+            g = 1 << (12 - plan[-1][0])
+            tops = [k for k in kernel_names(lambda: bc_ntt.lde(d, o, log_n, cols, log_b)) if "top_kernel" in k]
+            assert len(tops) == 1
+            assert ("top_kernel_tc" in tops[0]) == (log_b <= 4 and 4 * cols >= 3 * g * -(-cols // g)), (cols, tops)
     finally:
         bc_ntt.plan_table_clear()
         if old:
@@ -85,23 +90,20 @@ def test_lde_top_windows(gpu_ctx, plan, log_b):
 
 def test_chains_in_a_graph_and_on_two_streams(gpu_ctx):
     """Kernels of one call overlap each other's start: repeated calls that read the previous call's output, two
-    streams at once, and a captured graph give what single calls give."""
+    streams at once, and a captured graph give the canonical inputs back."""
     import torch
 
     import bc_ntt
 
     log_n, cols = 16, 16
     n = 1 << log_n
-    x = to_dev(raw_u64(np.random.default_rng(3), cols * n))
+    words = raw_u64(np.random.default_rng(3), cols * n)
+    x, want = to_dev(words), words % np.uint64(bc_ntt.P)
 
     def there_and_back(a, b):
         bc_ntt.batch_ntt_internal(a.data_ptr(), b.data_ptr(), log_n, cols, n, n, False, False, 0, 0)
         bc_ntt.batch_ntt_internal(b.data_ptr(), a.data_ptr(), log_n, cols, n, n, True, True, 0, 0)
 
-    a0, b0 = x.clone(), torch.empty_like(x)
-    there_and_back(a0, b0)
-    torch.cuda.synchronize()
-    want = to_host(a0)
     streams = [torch.cuda.Stream() for _ in range(2)]
     bufs = [(x.clone(), torch.empty_like(x)) for _ in streams]
     torch.cuda.synchronize()
@@ -121,6 +123,53 @@ def test_chains_in_a_graph_and_on_two_streams(gpu_ctx):
     torch.cuda.synchronize()
     assert np.array_equal(to_host(a), want)
     assert bc_ntt.wait_status() == 0
+
+
+@pytest.mark.parametrize("plan,log_b", [("2 8 8 8 1", 2), ("2 10 4 12 1", 1), ("2 4 8 9 1", 3)])
+def test_lde_chains_in_a_graph_and_on_two_streams(gpu_ctx, plan, log_b):
+    """The same for the fused LDE's kernels, the first of which leave their values in the last coset's block: both
+    streams and the graph give the oracle's extension, over and over."""
+    import torch
+
+    import bc_ntt
+    import oracle
+
+    log_n = sum(int(k) for k in plan.split()[1::2])
+    n, cols = 1 << log_n, 16 if log_n < 20 else 2
+    old = bc_ntt.plan_table_export()
+    words = [raw_u64(np.random.default_rng(s), cols * n) for s in range(2)]
+    want = [np.asarray(oracle.lde(w, log_n, cols, n, log_b, threads=8)) for w in words]
+    xs = [to_dev(w) for w in words]
+    try:
+        bc_ntt.plan_table_import(f"{log_n} {log_b} {plan}\n")
+        names = kernel_names(lambda: bc_ntt.lde(xs[0], torch.empty(cols * n << log_b, dtype=torch.int64, device="cuda"),
+                                                log_n, cols, log_b))
+        assert len(names) == 3 and all("kernel_tc<" in k for k in names), names
+        streams = [torch.cuda.Stream() for _ in xs]
+        outs = [torch.zeros(cols * n << log_b, dtype=torch.int64, device="cuda") for _ in xs]
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for s, x, o in zip(streams, xs, outs):
+                with torch.cuda.stream(s):
+                    bc_ntt.lde(x, o, log_n, cols, log_b)
+        torch.cuda.synchronize()
+        for o, w in zip(outs, want):
+            assert np.array_equal(to_host(o), w)
+            o.zero_()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for x, o in zip(xs, outs):
+                bc_ntt.lde(x, o, log_n, cols, log_b)
+        for _ in range(3):
+            g.replay()
+        torch.cuda.synchronize()
+        for o, w in zip(outs, want):
+            assert np.array_equal(to_host(o), w)
+        assert bc_ntt.wait_status() == 0
+    finally:
+        bc_ntt.plan_table_clear()
+        if old:
+            bc_ntt.plan_table_import(old)
 
 
 @pytest.mark.parametrize("log_n,log_b", [(13, 1), (13, 2), (14, 1), (15, 3), (18, 1)])

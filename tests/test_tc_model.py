@@ -28,8 +28,8 @@ def fold(d):
 
 def test_fold_digits():
     rnd = random.Random(1)
-    top = 128 * 255 * 255
-    cases = [[top] * 8, [0] * 8, [0] * 4 + [255] * 4, [255] * 8, [0] * 4 + [255, 255, 255, 256]]
+    top = 256 * 255 * 255  # 32 words a row
+    cases = [[top] * 8, [128 * 255 * 255] * 8, [0] * 8, [0] * 4 + [255] * 4, [255] * 8, [0] * 4 + [255, 255, 255, 256]]
     cases += [[rnd.choice((0, 1, 255, 256, top, rnd.randint(0, top))) for _ in range(8)] for _ in range(4000)]
     for d in cases:
         got = fold(d)

@@ -13,7 +13,7 @@ import numpy as np
 import pytest
 
 import oracle
-from conftest import raw_u64, to_dev, to_host
+from conftest import kernel_names, raw_u64, to_dev, to_host
 
 DIRECT_SHAPES = [(4, 8), (5, 8), (6, 8), (7, 8), (8, 8), (9, 8), (10, 4)]
 # "" = built-in knobs (resident tables where they fit); then top_mode PREFETCH, REFILL; then top_walk 2
@@ -35,6 +35,8 @@ def _run_plans(log_n, cols, passes, seed):
             bc_ntt.plan_table_import("".join(f"{log_n} {b} {passes}{knobs}\n" for b in (1, 3)))
             for log_b in (1, 3):
                 out = torch.empty(((1 << log_b) * cols) << log_n, dtype=torch.int64, device="cuda")
+                top = "lde_top_kernel<" + ",".join(passes.split()[1:3]) + ">"
+                assert top in kernel_names(lambda: bc_ntt.lde(d, out, log_n, cols, log_b))
                 bc_ntt.lde(d, out, log_n, cols, log_b)
                 torch.cuda.synchronize()
                 np.testing.assert_array_equal(to_host(out), expected[log_b],

@@ -59,25 +59,29 @@ def test_plan_table_roundtrip_and_validation(gpu_ctx):
     assert bc_ntt.plan_table_export() == ""
 
 
+@pytest.mark.parametrize("log_n,split,integer", [(17, "5 8 12 1", False), (14, "5 8 9 1", True)])
 @pytest.mark.parametrize("knobs", ["k 1 0 0 0 0", "k 32 2 0 0 0", "k 0 16 2 0 0", "k 0 0 3 0 0", "k 0 4 0 2 0",
                                    "k 0 0 0 1 3", "k 8 0 0 0 2", "k 4 2 3 2 3"])
-def test_plan_knobs_stay_exact(gpu_ctx, knobs):
+def test_plan_knobs_stay_exact(gpu_ctx, knobs, log_n, split, integer):
     """Every launch knob the autotuner may pick -- column walks, top-window table mode and double-buffering, pass
     occupancy -- gives the oracle's result, for a fused LDE with an 8-column top window (where double-buffering
-    applies) and for a plain NTT."""
+    applies) and for a plain NTT.  The first split runs on the tensor cores, which know the walks only; 5 columns do
+    not fill the second one's 9-bit tiles, so that the integer kernels run with all of the knobs."""
     import bc_ntt
     import torch
 
     bc_ntt.plan_table_clear()
-    bc_ntt.plan_table_import(f"17 1 2 5 8 12 1 {knobs}\n17 2 2 5 8 12 1 {knobs}\n17 0 2 5 8 12 1 {knobs}\n")
+    bc_ntt.plan_table_import("".join(f"{log_n} {b} 2 {split} {knobs}\n" for b in (0, 1, 2)))
     assert knobs in bc_ntt.plan_table_export()
     rng = np.random.default_rng(31)
-    log_n, cols = 17, 5
+    cols = 5
     n = 1 << log_n
     x = raw_u64(rng, cols * n)
     d = to_dev(x)
     for log_b in (1, 2):
         out = torch.empty(((1 << log_b) * cols) << log_n, dtype=torch.int64, device="cuda")
+        names = kernel_names(lambda: bc_ntt.lde(d, out, log_n, cols, log_b))
+        assert len(names) == 3 and all(("kernel_tc<" in k) != integer for k in names), names
         bc_ntt.lde(d, out, log_n, cols, log_b)
         torch.cuda.synchronize()
         np.testing.assert_array_equal(to_host(out), oracle.lde(x, log_n, cols, n, log_b, threads=8),
