@@ -25,6 +25,7 @@ from __future__ import annotations
 import argparse
 import json
 import os
+import re
 import sys
 import threading
 import time
@@ -58,21 +59,54 @@ def l2_note() -> str:
     return f"inputs {fmt(n_in)} and outputs {fmt(n_out)}; inputs fit in L2 (a small case, not the bench workload)"
 
 
-def measured_traffic(log_n: int, log_blowup: int, cols: int):
-    """DRAM bytes of one top-window launch from the committed ncu summary, scaled to `cols` columns, and the
-    ALU / FMA pipe utilisation (% of peak) of that capture: (bytes, alu_pct, fma_pct), Nones if absent."""
+def profiled_record(log_n: int, log_blowup: int):
+    """The committed ncu summary of the fused LDE's top-window kernel for this size, as a dict (`kernel`: the
+    profiled one); empty if absent."""
     path = os.path.join(ROOT, "profiles", f"lde_top_kernel_traffic_logn{log_n}_blowup{1 << log_blowup}.txt")
     try:
         for line in open(path):
             if line.startswith("kernel="):
                 kv = dict(tok.split("=", 1) for tok in line.split())
                 if int(kv["log_n"]) == log_n and int(kv["log_blowup"]) == log_blowup:
-                    byts = round((int(kv["dram_read"]) + int(kv["dram_write"])) * cols / int(kv["cols"]))
-                    alu, fma = kv.get("alu_pipe_pct"), kv.get("fma_pipe_pct")
-                    return byts, float(alu) if alu else None, float(fma) if fma else None
+                    return kv
     except OSError:
         pass
-    return None, None, None
+    return {}
+
+
+def measured_traffic(log_n: int, log_blowup: int, cols: int):
+    """DRAM bytes of one top-window launch from the committed ncu summary, scaled to `cols` columns, and the
+    ALU / FMA pipe utilisation (% of peak) of that capture: (bytes, alu_pct, fma_pct), Nones if absent."""
+    kv = profiled_record(log_n, log_blowup)
+    if not kv:
+        return None, None, None
+    byts = round((int(kv["dram_read"]) + int(kv["dram_write"])) * cols / int(kv["cols"]))
+    alu, fma = kv.get("alu_pipe_pct"), kv.get("fma_pipe_pct")
+    return byts, float(alu) if alu else None, float(fma) if fma else None
+
+
+def captured_kernels(launch):
+    """Names, with template arguments, of the kernels that launch(stream handle) enqueues, in order, read from a
+    graph it is captured into (nothing runs); None where that cannot be read."""
+    try:
+        import torch
+        from cuda.bindings import driver
+
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g):
+            launch(torch.cuda.current_stream().cuda_stream)
+        graph = driver.CUgraph(g.raw_cuda_graph())
+        _, _, count = driver.cuGraphGetNodes(graph)
+        _, nodes, _ = driver.cuGraphGetNodes(graph, count)
+        names = []
+        for node in nodes:
+            p = driver.cuGraphKernelNodeGetParams(node)[1]
+            name = (driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))[1].decode()
+            m = re.search(r"\d([a-z_]+)I((?:L[bij]\d+E)+)E", name)
+            names.append(f"{m[1]}<{','.join(re.findall(r'L[bij](\d+)E', m[2]))}>" if m else name)
+        return names
+    except Exception:  # bindings without these calls, or another kind of node
+        return None
 
 
 class ClockSampler:
@@ -450,7 +484,7 @@ def run_ours(args, rank, world):
     bit_exact_vs_plain = bool(torch.equal(ref_sum, out))
     del ref_sum
 
-    # the integer roofline first, on a GPU that has not yet run at full power for long
+    # the integer kernels' round loop first, on a GPU that has not yet run at full power for long
     peak_bfly, peak_ms, peak_clocks = butterfly_peak()
     with ClockSampler(int(os.environ.get("LOCAL_RANK", "0"))) as clk:
         total_ms, per = time_steps(fused, args.steps, args.warmup, world, stream)
@@ -486,28 +520,36 @@ def run_ours(args, rank, world):
     # top window read+write every coset
     col_bytes = 8 * n * COLS
     npass = (nk.value + 1) // 2 if nk.value else 1
-    kernels = ([(f"lde inverse pass {i} (b2n)", 2 * col_bytes) for i in range(npass - 1)]
-               + [("lde_top_kernel (inverse top window, scale, forward top window, all cosets)",
-                   (1 + B) * col_bytes)]
-               + [(f"lde forward pass {i} (n2b, all cosets)", 2 * B * col_bytes) for i in range(npass - 1)])
+    kernels = ([(f"inverse pass {i} (b2n)", 2 * col_bytes) for i in range(npass - 1)]
+               + [("inverse top window, scale, forward top window, all cosets", (1 + B) * col_bytes)]
+               + [(f"forward pass {i} (n2b, all cosets)", 2 * B * col_bytes) for i in range(npass - 1)])
+    ran = captured_kernels(lambda s: L.bc_lde_fused(xp, op, LOG_N, COLS, n, n, COLS * n, LOG_BLOWUP, s))
+    if not ran or len(ran) != len(kernels):
+        ran = [None] * len(kernels)
     roofline = None
-    traffic, alu_pct, fma_pct = measured_traffic(LOG_N, LOG_BLOWUP, COLS)
     windows = plan_windows(LOG_N, LOG_BLOWUP)
     kbfly = lde_kernel_butterflies(windows, LOG_N, COLS, LOG_BLOWUP) if windows else None
     if kern_ms and len(kern_ms) == len(kernels):
         dom = max(range(len(kern_ms)), key=lambda i: kern_ms[i])
-        name, byts = kernels[dom]
+        role, byts = kernels[dom]
+        name = f"{ran[dom]} ({role})" if ran[dom] else role
         achieved = byts / (kern_ms[dom] / 1e3) / 1e9
-        top = "lde_top_kernel" in name
+        # DRAM traffic and pipe shares only from a capture of the kernel that ran
+        record = profiled_record(LOG_N, LOG_BLOWUP)
+        profiled = bool(record) and record["kernel"] == ran[dom]
+        traffic, alu_pct, fma_pct = measured_traffic(LOG_N, LOG_BLOWUP, COLS) if profiled else (None, None, None)
+        on_tc = ran[dom] is not None and "kernel_tc" in ran[dom]
         # The HBM roofline of the kernel's algorithmic bytes (achieved / peak / frac) is reported as the contract
         # asks, but it does not bound these kernels: (1 + B) (n / 2) log n butterflies of 64-bit modular arithmetic
-        # on 32-bit integer pipes do.  `limiter` is that roofline: butterflies per second of the kernel against
-        # the same round arithmetic run from registers (bc_butterfly_peak, measured in this run).
-        roofline = {"bound": "int32 issue", "kernel": name, "achieved": round(achieved, 1), "peak": peak,
+        # do.  The integer kernels' ceiling is their own round arithmetic run from registers (bc_butterfly_peak,
+        # measured in this run).  The tensor-core kernels exceed that loop; what bounds them is the issue of the
+        # digit folds and power multiplications, and `limiter` gives the issue slots and pipes of the capture.
+        roofline = {"bound": "instruction issue" if on_tc else "int32 issue", "kernel": name,
+                    "achieved": round(achieved, 1), "peak": peak,
                     "unit": "GB/s", "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                     "hbm_frac_note": "achieved/peak/frac: HBM roofline of the algorithmic bytes; see limiter",
                     "spec_frac": round(achieved / SPEC_HBM_GBS, 4),
-                    "traffic": traffic if top else None,
+                    "traffic": traffic,
                     "traffic_unit": "bytes per launch (ncu dram read+write, scaled from the profiled case)",
                     "kernel_ms": [round(v, 3) for v in kern_ms],
                     "step_algorithmic_frac": round(8 * n * COLS * (1 + B) / (ms_per_step / 1e3) / 1e9 / peak, 4)}
@@ -515,18 +557,24 @@ def run_ours(args, rank, world):
             rates = [b / (t / 1e3) / 1e9 for b, t in zip(kbfly, kern_ms)]
             step_rate = sum(kbfly) / (ms_per_step / 1e3) / 1e9
             roofline["limiter"] = {
-                "bound": "int32 issue", "unit": "G butterflies/s", "kernel": name,
-                "achieved": round(rates[dom], 1), "peak": round(peak_bfly, 1),
-                "frac": round(rates[dom] / peak_bfly, 4),
-                "per_kernel_achieved": [round(r, 1) for r in rates],
-                "step_achieved": round(step_rate, 1), "step_frac": round(step_rate / peak_bfly, 4),
+                "bound": roofline["bound"], "unit": "G butterflies/s", "kernel": name,
+                "achieved": round(rates[dom], 1),
+                # the tensor-core kernels have no such peak: null, not a fraction of a loop they do not run
+                "peak": None if on_tc else round(peak_bfly, 1),
+                "frac": None if on_tc else round(rates[dom] / peak_bfly, 4),
+                "per_kernel_achieved": [round(r, 1) for r in rates], "kernels": ran,
+                "step_achieved": round(step_rate, 1),
+                "step_frac": None if on_tc else round(step_rate / peak_bfly, 4),
                 "butterflies_per_step": sum(kbfly), "plan_windows": windows,
-                "peak_source": f"bc_butterfly_peak: the kernels' radix-16 round arithmetic from registers, every "
-                               f"resident thread slot, best of 5 launches of {peak_ms:.1f} ms, this run",
-                "peak_clocks": peak_clocks,
+                "integer_loop": round(peak_bfly, 1),
+                "integer_loop_source": f"bc_butterfly_peak: the integer kernels' radix-16 round arithmetic from "
+                                       f"registers, every resident thread slot, best of 5 launches of {peak_ms:.1f} "
+                                       f"ms, this run",
+                "integer_loop_clocks": peak_clocks,
+                "issue_active_pct": float(record["issue_active_pct"]) if profiled else None,
                 "alu_pipe_pct": alu_pct, "fma_pipe_pct": fma_pct,
-                "pipe_source": "ncu of the top-window kernel and of the round loop, "
-                               "profiles/int32_roofline_butterfly_peak_and_lde_kernels_8cols_logn22_blowup2.md"}
+                "tensor_pipe_pct": float(record["tensor_pipe_pct"]) if profiled else None,
+                "pipe_source": f"ncu of that kernel, profiles/{record['source']}" if profiled else None}
 
     # end to end through the C ABI with host buffers: bc_lde_host takes pinned host input and writes pinned
     # host output every step, overlapping chunked copy-in / transform / copy-out on three streams
