@@ -215,63 +215,63 @@ bool build_lde_steps(const Plan &pl, const uint64_t *in, uint64_t *out, uint32_t
       st.grid = dim3((uint32_t)tiles, (uint32_t)gy);
       steps.push_back(st);
     } else {
-    const uint32_t nb = 1u << log_blowup;
-    // forward power tables: all resident if they fit with two CTAs per SM, else
-    // two slots fed ahead by cp.async from the precomputed ones, else refilled
-    const bool direct = top_direct(K, C); // top_body_direct: short-round-on-top tables, one tile
-    p.fwd_tables = top_power_tables((uint32_t)K, log_blowup, false, direct);
-    p.inv_table = top_power_tables((uint32_t)K, log_blowup, true, direct);
-    auto fits = [&](uint32_t tables) {
-      return (size_t)top_smem_words(tile, K, tables) * sizeof(uint64_t) <= TOP_RESIDENT_SMEM_MAX;
-    };
-    uint32_t slots = 1;
-    const bool can_prefetch = p.fwd_tables && K >= 4 && fits(2);
-    const uint8_t mode = pl.knobs.top_mode;
-    if (mode == TOP_MODE_REFILL) {
-      p.fwd_mode = TOP_TABLES_REFILL;
-    } else if (mode == TOP_MODE_PREFETCH && can_prefetch) {
-      p.fwd_mode = TOP_TABLES_PREFETCH;
-      slots = 2;
-    } else if (fits(nb)) {
-      p.fwd_mode = TOP_TABLES_RESIDENT;
-      slots = nb;
-    } else if (can_prefetch) {
-      p.fwd_mode = TOP_TABLES_PREFETCH;
-      slots = 2;
-    } else {
-      p.fwd_mode = TOP_TABLES_REFILL;
-    }
-    // two tiles (the next column group copied during this one) in the 8-column
-    // kernels with short transforms per tile (window bits x cosets <= 16: on
-    // B200 2^16 x 4096 columns, blowup 2, gains 13 %; 2^19 x 512, blowup 4,
-    // loses 2 %), when they fit and cost no resident CTA per SM
-    const size_t smem1 = (size_t)top_smem_words(tile, K, slots, 1) * sizeof(uint64_t);
-    const size_t smem2 = (size_t)top_smem_words(tile, K, slots, 2) * sizeof(uint64_t);
-    p.dbuf = 0;
-    const bool dbuf_allowed = !direct && C == 8 && p.fwd_mode != TOP_TABLES_PREFETCH && p.cols_per_cta > G &&
-                              smem2 <= TOP_RESIDENT_SMEM_MAX;
-    if (pl.knobs.top_dbuf == 2) {
-      p.dbuf = dbuf_allowed ? 1 : 0;
-    } else if (pl.knobs.top_dbuf == 0 && dbuf_allowed && (uint32_t)K * nb <= 16) {
-      const int n2 = top_ctas_per_sm(K, C, st.threads, smem2);
-      p.dbuf = (n2 > 0 && n2 >= top_ctas_per_sm(K, C, st.threads, smem1)) ? 1 : 0;
-    }
-    st.smem = p.dbuf ? smem2 : smem1;
-    // the scale factors once per CTA in shared memory, when the CTA walks more
-    // than one column group and the table costs no resident CTA per SM
-    p.scale_off = 0;
-    if (K >= 4 && p.cols_per_cta > G) {
-      const size_t with = st.smem + (size_t)tile * sizeof(uint64_t);
-      if (with <= TOP_RESIDENT_SMEM_MAX &&
-          top_ctas_per_sm(K, C, st.threads, with) >= top_ctas_per_sm(K, C, st.threads, st.smem)) {
-        p.scale_off = (uint32_t)(st.smem / sizeof(uint64_t));
-        st.smem = with;
+      const uint32_t nb = 1u << log_blowup;
+      // forward power tables: all resident if they fit with two CTAs per SM, else
+      // two slots fed ahead by cp.async from the precomputed ones, else refilled
+      const bool direct = top_direct(K, C); // top_body_direct: short-round-on-top tables, one tile
+      p.fwd_tables = top_power_tables((uint32_t)K, log_blowup, false, direct);
+      p.inv_table = top_power_tables((uint32_t)K, log_blowup, true, direct);
+      auto fits = [&](uint32_t tables) {
+        return (size_t)top_smem_words(tile, K, tables) * sizeof(uint64_t) <= TOP_RESIDENT_SMEM_MAX;
+      };
+      uint32_t slots = 1;
+      const bool can_prefetch = p.fwd_tables && K >= 4 && fits(2);
+      const uint8_t mode = pl.knobs.top_mode;
+      if (mode == TOP_MODE_REFILL) {
+        p.fwd_mode = TOP_TABLES_REFILL;
+      } else if (mode == TOP_MODE_PREFETCH && can_prefetch) {
+        p.fwd_mode = TOP_TABLES_PREFETCH;
+        slots = 2;
+      } else if (fits(nb)) {
+        p.fwd_mode = TOP_TABLES_RESIDENT;
+        slots = nb;
+      } else if (can_prefetch) {
+        p.fwd_mode = TOP_TABLES_PREFETCH;
+        slots = 2;
+      } else {
+        p.fwd_mode = TOP_TABLES_REFILL;
       }
-    }
-    const uint64_t gy = (num_cols + p.cols_per_cta - 1) / p.cols_per_cta;
-    if (gy > 65535 || tiles > 0x7fffffffull) return false;
-    st.grid = dim3((uint32_t)tiles, (uint32_t)gy);
-    steps.push_back(st);
+      // two tiles (the next column group copied during this one) in the 8-column
+      // kernels with short transforms per tile (window bits x cosets <= 16: on
+      // B200 2^16 x 4096 columns, blowup 2, gains 13 %; 2^19 x 512, blowup 4,
+      // loses 2 %), when they fit and cost no resident CTA per SM
+      const size_t smem1 = (size_t)top_smem_words(tile, K, slots, 1) * sizeof(uint64_t);
+      const size_t smem2 = (size_t)top_smem_words(tile, K, slots, 2) * sizeof(uint64_t);
+      p.dbuf = 0;
+      const bool dbuf_allowed = !direct && C == 8 && p.fwd_mode != TOP_TABLES_PREFETCH && p.cols_per_cta > G &&
+                                smem2 <= TOP_RESIDENT_SMEM_MAX;
+      if (pl.knobs.top_dbuf == 2) {
+        p.dbuf = dbuf_allowed ? 1 : 0;
+      } else if (pl.knobs.top_dbuf == 0 && dbuf_allowed && (uint32_t)K * nb <= 16) {
+        const int n2 = top_ctas_per_sm(K, C, st.threads, smem2);
+        p.dbuf = (n2 > 0 && n2 >= top_ctas_per_sm(K, C, st.threads, smem1)) ? 1 : 0;
+      }
+      st.smem = p.dbuf ? smem2 : smem1;
+      // the scale factors once per CTA in shared memory, when the CTA walks more
+      // than one column group and the table costs no resident CTA per SM
+      p.scale_off = 0;
+      if (K >= 4 && p.cols_per_cta > G) {
+        const size_t with = st.smem + (size_t)tile * sizeof(uint64_t);
+        if (with <= TOP_RESIDENT_SMEM_MAX &&
+            top_ctas_per_sm(K, C, st.threads, with) >= top_ctas_per_sm(K, C, st.threads, st.smem)) {
+          p.scale_off = (uint32_t)(st.smem / sizeof(uint64_t));
+          st.smem = with;
+        }
+      }
+      const uint64_t gy = (num_cols + p.cols_per_cta - 1) / p.cols_per_cta;
+      if (gy > 65535 || tiles > 0x7fffffffull) return false;
+      st.grid = dim3((uint32_t)tiles, (uint32_t)gy);
+      steps.push_back(st);
     }
   }
   // C: forward passes below the top window for all cosets (column groups with prefix brev(k))

@@ -85,8 +85,8 @@ constexpr uint32_t BATCH_THREADS = 256;
 // What the launch bounds, BATCH_SMEM_BYTES and the tensor memory (256 of 512
 // columns each) allow.  Not asked of the occupancy calculator: for kernels that
 // allocate tensor memory it answers 1 whatever their share (192 small jobs:
-// 2336 us with one CTA an SM, 1447 with two).  The schedule needs no particular number: items
-// are taken in order by CTAs that run.
+// 2212 us with one CTA an SM, 1348 with two).  The schedule needs no particular
+// number: items are taken in order by CTAs that run.
 constexpr int BATCH_CTAS_PER_SM = 2;
 // largest bodies: the top window of 12 bits with one forward table, and the
 // tensor-core top window of 10 bits (two CTAs an SM either way)

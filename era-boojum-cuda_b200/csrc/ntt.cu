@@ -287,7 +287,8 @@ static bool fit_split(int low, uint32_t log_n, uint32_t cols, bool whole_rounds,
   for (int any = whole_rounds ? 0 : 1; any < 2; any++)
     for (int k = low + 1; k <= 12; k++) {
       const int top = (int)log_n - k;
-      if ((top == 4 || top == 8 || top == 10 || (any && (top == 5 || top == 9))) && tc_window_ok(k, 0, cols, true, true)) {
+      const bool has = top == 4 || top == 8 || top == 10 || (any && (top == 5 || top == 9));
+      if (has && tc_window_ok(k, 0, cols, true, true)) {
         const Knobs knobs = pl.knobs;
         pl = two_pass(top, k);
         pl.knobs = knobs;

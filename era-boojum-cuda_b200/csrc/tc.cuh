@@ -52,8 +52,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)_
 
 // Programmatic dependent launch: the kernels of one call overlap each other's
 // prologue (tables, matrices).  allow_next once the CTA has its tensor memory
-// (the next kernel's CTAs hold theirs while they wait); a kernel touches what its predecessor wrote (or reads) only after wait_previous, which
-// returns when the predecessor has completed and its stores are visible.
+// (the next kernel's CTAs hold theirs while they wait); a kernel touches what its
+// predecessor wrote (or reads) only after wait_previous, which returns when the
+// predecessor has completed and its stores are visible.
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -146,7 +147,8 @@ __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c)
 }
 
 // sum_j d[j] 2^(8j) (mod p) as a u64, for d[j] <= 256 * 255^2 < 2^24 (32 words
-// a row; 16 give half of that).  Pairs first: p = d + 2^8 d' < 2^32; L = p0 + 2^16 p1 and H = p2 + 2^16 p3 < 2^49.  With
+// a row; 16 give half of that).  Pairs first: p = d + 2^8 d' < 2^32; L = p0 +
+// 2^16 p1 and H = p2 + 2^16 p3 < 2^49.  With
 // H = h0 + h1 2^32: L + h0 2^32 + h1 2^64 = (L + h1 EPS) + h0 2^32, where
 // L + h1 EPS < 2^50, so one carry can leave the top word and the fold of its
 // EPS cannot carry again (the top word wrapped to less than 2^18).

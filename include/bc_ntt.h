@@ -29,7 +29,7 @@ extern "C" {
 #endif
 
 /* Replaces Context::create (src/context.rs:171-282).  Builds this library's
- * twiddle and power tables on the CURRENT device (about 1.7 MB); every other
+ * twiddle and power tables on the CURRENT device (about 15 MB); every other
  * call on that device requires it and returns cudaErrorInitializationError
  * without it.  The two counts keep the reference's bounds check (<= 24); the
  * table split itself is fixed.  Idempotent; thread-safe. */
