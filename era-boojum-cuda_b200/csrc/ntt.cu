@@ -330,7 +330,7 @@ Plan fit_ntt_plan(Plan pl, uint32_t log_n, uint32_t cols, bool b2n, bool inverse
   // forward transform of a coset.  Columns that do not fill a tile are nothing
   // to it, and the splits are those that suit it best (3 x 2^16 inverse: 16 us
   // as 8 + 8, 20 as 5 + 11; of a coset, 12 x 2^13: 20 as 5 + 8, 25 as 4 + 9; 3 x
-  // 2^21: 159 as 9 + 12, 186 as 4 + 8 + 9), with three CTAs an SM in low windows
+  // 2^21: 159 as 9 + 12, 170 as 4 + 8 + 9), with three CTAs an SM in low windows
   // of 9..11 bits (33 x 2^17: 120 against 131).
   if (b2n != inverse && (inverse || coset)) {
     if (!two || log_n > 22) return pl;
