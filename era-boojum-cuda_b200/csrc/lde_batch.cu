@@ -321,6 +321,26 @@ size_t schedule_bytes(size_t n_records, size_t n_items) {
          round256(n_records * sizeof(BatchRecord)) + n_items * sizeof(uint64_t);
 }
 
+// A job's kernels as work of the persistent kernel; false when that does not carry one of them.
+bool build_batch_steps(const Plan &pl, const bc_lde_job &jb, std::vector<LdeStep> &steps) {
+  if (!build_lde_steps(pl, jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols, jb.stride_in, jb.stride_out, jb.coset_stride,
+                       jb.log_blowup, true, 16, 16, steps))
+    return false;
+  for (const LdeStep &st : steps)
+    if (!(st.tc ? batch_tc_shape_supported(tc_shape_id(st.top, st.b2n, !st.top && st.pass.lb == 0, st.K))
+                : batch_shape_supported(shape_id(st.top, st.b2n, st.K, st.C))) ||
+        st.threads != BATCH_THREADS || st.smem > BATCH_SMEM_BYTES || st.grid.x >= (1u << 28) ||
+        st.grid.y >= (1u << 20) || (!st.top && st.pass.inverse != (uint32_t)st.b2n)) // the kernel carries LDE passes only
+      return false;
+  return true;
+}
+
+uint64_t items_of(const std::vector<LdeStep> &steps) {
+  uint64_t n = 0;
+  for (const LdeStep &st : steps) n += (uint64_t)st.grid.x * st.grid.y;
+  return n;
+}
+
 // Records and items of a batch, in dependency order (host side).
 // standalone_min_ctas > 0: a job whose every kernel, launched on its own, has
 // at least that many CTAs goes to `standalone` (its fused-LDE steps in order)
@@ -331,6 +351,7 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
                      std::vector<uint64_t> &items, uint32_t standalone_min_ctas = 0,
                      std::vector<LdeStep> *standalone = nullptr, size_t max_bytes = 0) {
   std::vector<std::vector<LdeStep>> steps(n_jobs);
+  std::vector<char> fixed(n_jobs, 0);
   size_t max_depth = 0;
   for (uint32_t j = 0; j < n_jobs; j++) {
     const bc_lde_job &jb = jobs[j];
@@ -350,33 +371,37 @@ cudaError_t schedule(const bc_lde_job *jobs, uint32_t n_jobs, std::vector<BatchR
       }
     }
     // the call's plan, or the built-in one when that uses a window shape this kernel does not carry
-    auto build = [&](const Plan &pl) {
-      if (!build_lde_steps(pl, jb.evals_bitrev, jb.out, jb.log_n, jb.num_cols, jb.stride_in, jb.stride_out,
-                           jb.coset_stride, jb.log_blowup, true, 16, 16, steps[j]))
-        return false;
-      for (const LdeStep &st : steps[j])
-        if (!(st.tc ? batch_tc_shape_supported(tc_shape_id(st.top, st.b2n, !st.top && st.pass.lb == 0, st.K))
-                    : batch_shape_supported(shape_id(st.top, st.b2n, st.K, st.C))) ||
-            st.threads != BATCH_THREADS ||
-            st.smem > BATCH_SMEM_BYTES || st.grid.x >= (1u << 28) || st.grid.y >= (1u << 20) ||
-            (!st.top && st.pass.inverse != (uint32_t)st.b2n)) // the kernel carries LDE passes only
-          return false;
-      return true;
-    };
-    if (!build(call_plan(jb.log_n, jb.log_blowup, jb.num_cols)) && !build(default_plan(jb.log_n)))
+    bool own = false;
+    if (!build_batch_steps(call_plan(jb.log_n, jb.log_blowup, jb.num_cols, &own), jb, steps[j]) &&
+        !build_batch_steps(default_plan(jb.log_n), jb, steps[j]))
       return cudaErrorInvalidConfiguration;
-    max_depth = std::max(max_depth, steps[j].size());
+    fixed[j] = own;
   }
-  if (max_bytes) {
+  auto fits = [&] {
     uint64_t n_recs = 0, n_items = 0;
-    for (uint32_t j = 0; j < n_jobs; j++)
-      for (const LdeStep &st : steps[j]) {
-        n_recs++;
-        n_items += (uint64_t)st.grid.x * st.grid.y;
+    for (const auto &s : steps) {
+      n_recs += s.size();
+      n_items += items_of(s);
+    }
+    return n_items <= max_bytes / sizeof(uint64_t) && schedule_bytes(n_recs, n_items) <= max_bytes;
+  };
+  if (max_bytes && !fits()) {
+    // Not with these plans: the two-pass split of fewest work items for every
+    // job whose plan is not the caller's own (280 jobs of 8 columns of 2^21,
+    // blowup 8, need 26.5 MB as 10 + 11 bits, 16.2 as 9 + 12).
+    std::vector<LdeStep> alt;
+    for (uint32_t j = 0; j < n_jobs; j++) {
+      if (fixed[j] || steps[j].empty()) continue;
+      for (int top : {4, 5, 8, 9, 10}) {
+        const int low = (int)jobs[j].log_n - top;
+        if (low >= 8 && low <= 12 && build_batch_steps(two_pass(top, low), jobs[j], alt) &&
+            items_of(alt) < items_of(steps[j]))
+          steps[j].swap(alt);
       }
-    if (n_items > max_bytes / sizeof(uint64_t) || schedule_bytes(n_recs, n_items) > max_bytes)
-      return cudaErrorInvalidValue;
+    }
+    if (!fits()) return cudaErrorInvalidValue;
   }
+  for (const auto &s : steps) max_depth = std::max(max_depth, s.size());
   // big jobs first within every depth
   std::vector<uint32_t> order(n_jobs);
   for (uint32_t j = 0; j < n_jobs; j++) order[j] = j;

@@ -239,7 +239,7 @@ cudaError_t context_destroy_current() {
 }
 
 // ---------------------------------------------------------------- plans
-static Plan two_pass(int top, int low) {
+Plan two_pass(int top, int low) {
   Plan pl{};
   pl.npasses = 2;
   pl.pass[0] = {(uint8_t)top, (uint8_t)(top <= 9 ? 8 : top == 10 ? 4 : 2)};

@@ -68,13 +68,14 @@ int current_device();
 int sm_count();
 
 Plan default_plan(uint32_t log_n);
+Plan two_pass(int top, int low); // windows of `top` bits above `low` bits
 // The plan, or one that suits the columns (and kind of transform) better.
 Plan fit_plan(Plan pl, uint32_t log_n, uint32_t cols);
 Plan fit_ntt_plan(Plan pl, uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset);
 // The plan of an LDE and of a plain NTT on the current device (tune.cu): an
 // entry that the caller imported or autotuned, as it is; else the default entry
 // of the table or, without one, default_plan, either fitted to the call.
-Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols);
+Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols, bool *own = nullptr); // *own: it is the caller's
 Plan call_ntt_plan(uint32_t log_n, uint32_t cols, bool b2n, bool inverse, bool coset);
 bool plan_valid(const Plan &pl, uint32_t log_n);
 

@@ -132,8 +132,9 @@ static Entry entry_of(uint32_t log_n, uint32_t log_blowup) {
   return Entry{default_plan(log_n), true};
 }
 
-Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols) {
+Plan call_plan(uint32_t log_n, uint32_t log_blowup, uint32_t cols, bool *own) {
   const Entry en = entry_of(log_n, log_blowup);
+  if (own) *own = !en.fit;
   return en.fit ? fit_plan(en.plan, log_n, cols) : en.plan;
 }
 

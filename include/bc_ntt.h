@@ -232,7 +232,8 @@ cudaError_t bc_lde_batch_plan_destroy(bc_lde_batch_plan *plan);
  * cudaFree: the schedule goes into a fixed 16 MiB array inside this library,
  * which every GPU that loads the library holds until the process exits.  A
  * batch whose schedule does not fit (about two million 4096-element work
- * items) returns cudaErrorInvalidValue before its work items are built.  The
+ * items), also with other splits in place of built-in and default plans,
+ * returns cudaErrorInvalidValue before its work items are built.  The
  * first call on a device looks up the array's device address and the kernel's
  * occupancy and keeps them for the life of the process: they do not survive
  * cudaDeviceReset (or any other replacement of the device's primary context).

@@ -128,3 +128,40 @@ def test_noalloc_batch_holds_many_small_jobs(gpu_ctx, log_n, cols, jobs_per_batc
     ref = torch.empty_like(job[1])
     bc_ntt.lde(job[0], ref, log_n, cols, log_b)
     assert bool((outs == ref).all())
+
+
+def test_noalloc_batch_takes_other_splits_when_its_plans_do_not_fit(gpu_ctx):
+    """505 jobs of 33 columns of 2^17 need more than the array with the shipped table's split, less with another: the
+    batch is accepted and exact.  A plan that the caller imported is not replaced."""
+    import torch
+
+    import bc_ntt
+
+    log_n, cols, log_b, count = 17, 33, 1, 505
+    n = 1 << log_n
+    (job,), _ = _jobs(np.random.default_rng(4), [(log_n, cols, log_b)])
+    outs = torch.full((count, (cols * n) << log_b), 0x11, dtype=torch.int64, device="cuda")
+    arr = (bc_ntt.LdeJob * count)()
+    for i in range(count):
+        arr[i] = bc_ntt.LdeJob(job[0].data_ptr(), outs.data_ptr() + 8 * i * outs.shape[1], n, n, cols * n, log_n, cols,
+                               log_b, 0)
+
+    def run():
+        status = ctypes.c_uint32(0xFFFF)
+        rc = bc_ntt.lib().bc_lde_batch_noalloc(ctypes.cast(arr, ctypes.c_void_p), count,
+                                               torch.cuda.current_stream().cuda_stream, ctypes.byref(status))
+        return rc, status.value
+
+    try:
+        bc_ntt.plan_table_import(f"{log_n} {log_b} 2 5 8 12 1\n")
+        assert run()[0] == 1  # cudaErrorInvalidValue, nothing enqueued
+        bc_ntt.plan_table_clear()
+        assert bc_ntt.load_tuned_plans()
+        assert run() == (0, 0)
+        ref = torch.empty_like(job[1])
+        bc_ntt.lde(job[0], ref, log_n, cols, log_b)
+        assert all(bool((o == ref).all()) for o in outs)
+    finally:
+        bc_ntt.plan_table_clear()
+        del outs
+        torch.cuda.empty_cache()
